@@ -114,7 +114,8 @@ int wtq_append(const void *k, const void *v, int dtype, const int64_t k_strides[
  * history.  q: (B, Hq, D) of `dtype`, element strides {batch, head}; out:
  * same shape, own strides, same dtype (it may be a slice of a larger gathered
  * buffer).  Query head h reads kv head h / (Hq/Hkv).  num_splits <= 0 lets the
- * library choose.  The rotated query, the split-K partial states and the merge
+ * library choose (calls about the size of the chip then run as one kernel that
+ * does not touch the workspace).  The rotated query, the split-K partial states and the merge
  * live in `workspace` (wtq_decode_workspace_bytes); nothing else is allocated.
  * The first wtq_decode_counter_bytes() of the workspace must be zero on entry
  * and are zero again when the call's work completes.  Sequences of length 0
@@ -130,6 +131,16 @@ int wtq_decode(const void *q, int dtype, const int64_t q_strides[2], void *out,
                float scale, int B, int Hq, int Hkv, int D, int S, int P, int max_pages,
                int num_splits, void *workspace, size_t workspace_bytes, int32_t *status,
                void *stream);
+
+/* wtq_decode for callers that want to know first whether a workspace is needed:
+ * runs the call as ONE kernel without any, or returns WTQ_ERR_UNSUPPORTED with
+ * nothing launched where wtq_decode would take its split-K path (which calls do
+ * depends on sizes and alignment only). */
+int wtq_decode_direct(const void *q, int dtype, const int64_t q_strides[2], void *out,
+                      const int64_t out_strides[2], const wtq_side_t *k_side, const wtq_side_t *v_side,
+                      const int32_t *page_table, int64_t table_stride, const int32_t *seq_lens,
+                      float scale, int B, int Hq, int Hkv, int D, int S, int P, int max_pages,
+                      int32_t *status, void *stream);
 
 /* wtq_decode fused with the output exchange of KV-head tensor parallelism (no
  * counterpart in the reference, which has no multi-GPU form of this path).

@@ -56,6 +56,11 @@ _SIGNATURES = {
     "wtq_decode_workspace_bytes": (c_size_t, [c_int] * 7),
     "wtq_decode_counter_bytes": (c_size_t, [c_int, c_int]),
     "wtq_decode_auto_splits": (c_int, [c_int] * 8),
+    "wtq_decode_direct": (c_int, [c_void_p, c_int, ctypes.POINTER(c_int64), c_void_p,
+                                  ctypes.POINTER(c_int64), ctypes.POINTER(Side),
+                                  ctypes.POINTER(Side), c_void_p, c_int64, c_void_p, c_float,
+                                  c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p,
+                                  c_void_p]),
     "wtq_decode": (c_int, [c_void_p, c_int, ctypes.POINTER(c_int64), c_void_p,
                            ctypes.POINTER(c_int64), ctypes.POINTER(Side), ctypes.POINTER(Side),
                            c_void_p, c_int64, c_void_p, c_float, c_int, c_int, c_int, c_int, c_int,

@@ -44,6 +44,31 @@ bool fill_side(DecodeSideDev &d, const wtq_side_t &w, int D) {
   return w.pages && w.norms && w.Pi && w.centroids;
 }
 
+// Blocks per group when the call runs as one launch, else 0.
+int one_launch_cluster(const DecodeParams &p) {
+  return fused_eligible(p) && !force_generic() ? fused_cluster(p) : 0;
+}
+int one_launch(const DecodeParams &p, int cluster, const void *q, int dtype, const int64_t q_strides[2],
+               float scale, void *out, const int64_t out_strides[2], cudaStream_t stream) {
+  profile_mark_call(stream, true);
+  // (exp2 domain: log2(e) folded into the query)
+  const int rc = launch_decode_fused(p, q, dtype, q_strides, scale * 1.4426950408889634f, out, out_strides,
+                                     cluster, stream);
+  profile_mark_call(stream, false);
+  return rc;
+}
+void fill_call(DecodeParams &p, const wtq_side_t *k_side, const wtq_side_t *v_side,
+               const int32_t *page_table, int64_t table_stride, const int32_t *seq_lens, int B, int Hq,
+               int Hkv, int D, int S, int P, int max_pages, int32_t *status) {
+  fill_side(p.k, *k_side, D);
+  fill_side(p.v, *v_side, D);
+  p.page_table = page_table;
+  p.table_stride = table_stride;
+  p.seq_lens = seq_lens;
+  p.B = B; p.Hq = Hq; p.Hkv = Hkv; p.n_rep = Hq / Hkv; p.D = D; p.S = S; p.P = P;
+  p.max_pages = max_pages; p.status = status;
+}
+
 }  // namespace
 
 extern "C" size_t wtq_decode_counter_bytes(int B, int Hkv) {
@@ -160,8 +185,7 @@ static int decode_common(const void *q, int dtype, const int64_t q_strides[2], v
     return rc;
   if (B == 0) return WTQ_OK;
   DecodeParams p;
-  fill_side(p.k, *k_side, D);
-  fill_side(p.v, *v_side, D);
+  fill_call(p, k_side, v_side, page_table, table_stride, seq_lens, B, Hq, Hkv, D, S, P, max_pages, status);
   if (!workspace) return fail(WTQ_ERR_ARG, "wtq_decode: null workspace");
   const int splits = num_splits > 0 ? clamp_splits(num_splits, max_pages, S)
                                     : wtq_decode_auto_splits(B, Hq, Hkv, D, max_pages, S,
@@ -169,6 +193,10 @@ static int decode_common(const void *q, int dtype, const int64_t q_strides[2], v
   const size_t need = workspace_for(B, Hq, Hkv, D, splits);
   if (workspace_bytes < need)
     return fail(WTQ_ERR_WORKSPACE, "wtq_decode: workspace %zu < %zu bytes", workspace_bytes, need);
+
+  if (!exchange && num_splits <= 0)
+    if (const int cluster = one_launch_cluster(p))
+      return one_launch(p, cluster, q, dtype, q_strides, scale, out, out_strides, stream);
 
   const size_t rows = (size_t)B * Hq;
   p.work_counter = (int32_t *)workspace;
@@ -186,11 +214,7 @@ static int decode_common(const void *q, int dtype, const int64_t q_strides[2], v
   p.lut = (const uint32_t *)ws;
 
   p.q_rot = q_rot;
-  p.page_table = page_table;
-  p.table_stride = table_stride;
-  p.seq_lens = seq_lens;
-  p.B = B; p.Hq = Hq; p.Hkv = Hkv; p.n_rep = Hq / Hkv; p.D = D; p.S = S; p.P = P;
-  p.max_pages = max_pages; p.num_splits = splits; p.status = status;
+  p.num_splits = splits;
 
   MergeParams m;
   m.part_acc = p.part_acc; m.part_m = p.part_m; m.part_l = p.part_l;
@@ -252,6 +276,25 @@ extern "C" int wtq_decode(const void *q, int dtype, const int64_t q_strides[2], 
   return decode_common(q, dtype, q_strides, out, out_strides, nullptr, k_side, v_side, page_table,
                        table_stride, seq_lens, scale, B, Hq, Hkv, D, S, P, max_pages, num_splits,
                        workspace, workspace_bytes, status, stream);
+}
+
+extern "C" int wtq_decode_direct(const void *q, int dtype, const int64_t q_strides[2], void *out,
+                                 const int64_t out_strides[2], const wtq_side_t *k_side,
+                                 const wtq_side_t *v_side, const int32_t *page_table,
+                                 int64_t table_stride, const int32_t *seq_lens, float scale, int B,
+                                 int Hq, int Hkv, int D, int S, int P, int max_pages, int32_t *status,
+                                 void *stream) {
+  if (int rc = decode_validate(q, dtype, q_strides, out, out_strides, false, k_side, v_side, page_table,
+                               seq_lens, B, Hq, Hkv, D, S, P, max_pages))
+    return rc;
+  if (B == 0) return WTQ_OK;
+  DecodeParams p;
+  fill_call(p, k_side, v_side, page_table, table_stride, seq_lens, B, Hq, Hkv, D, S, P, max_pages, status);
+  const int cluster = one_launch_cluster(p);
+  if (!cluster)
+    return fail(WTQ_ERR_UNSUPPORTED, "wtq_decode_direct: this call is served by more than one launch and "
+                "needs a workspace (wtq_decode)");
+  return one_launch(p, cluster, q, dtype, q_strides, scale, out, out_strides, (cudaStream_t)stream);
 }
 
 extern "C" int wtq_decode_exchange(const void *q, int dtype, const int64_t q_strides[2],

@@ -88,6 +88,13 @@ int mma_chunk_tokens(int max_tokens, int splits);
 int launch_decode_mma(const DecodeParams &p, const MergeParams &m, cudaStream_t stream);
 int launch_mma_merge(const MergeParams &m, const int32_t *seq_lens, int B, int Hkv, int n_rep,
                      int chunk_tokens, int max_tokens, cudaStream_t stream);
+// One launch per call (wtq_decode_fused.cu): blocks per (sequence, kv head) group,
+// 0 where the split-K path is the better one; needs no workspace.
+bool fused_eligible(const DecodeParams &p);
+int fused_cluster(const DecodeParams &p);
+int launch_decode_fused(const DecodeParams &p, const void *q, int dtype, const int64_t q_strides[2],
+                        float q_scale, void *out, const int64_t out_strides[2], int cluster,
+                        cudaStream_t stream);
 // Tensor-core forms of the query rotation and of the chunk merge for calls with
 // thousands of rows (wtq_rows_mma.cu); the *_eligible functions say whether a
 // call qualifies (contiguous rows of 128, at least 4096 of them, 16-byte aligned
