@@ -8,7 +8,7 @@ from ctypes import c_float, c_int, c_int32, c_int64, c_size_t, c_void_p
 
 import torch
 
-from ._build import LIB
+from ._build import HOST, LIB
 
 WTQ_F32, WTQ_F16, WTQ_BF16 = 0, 1, 2
 ORDER_AUTO, ORDER_SEQUENTIAL, ORDER_INTERLEAVED16 = -1, 0, 1
@@ -125,6 +125,22 @@ def lib():
             fn.restype, fn.argtypes = res, args
         _lib = handle
     return _lib
+
+
+_host = None
+
+
+def host():
+    """The native host side of the operators (csrc/host.cpp)."""
+    global _host
+    if _host is None:
+        lib()                              # raises if the kernels are not built
+        if not os.path.exists(HOST):
+            raise BackendError(f"{HOST} is not built; see winnow_b200/_build.py")
+        from . import _host as module
+        module.set_error(BackendError)
+        _host = module
+    return _host
 
 
 def check(rc: int) -> None:

@@ -118,8 +118,9 @@ class PagedPackedCache:
         self.kq, self.vq = k_quant, v_quant
         self.head_dim = head_dim
         self.decode_backend = decode_backend
-        self._table = self._seq = self._refs = None
+        self._table = self._seq = None
         self.status = None
+        self._quants = None if pool.dense else (pa.Quantizer.from_tq(k_quant), pa.Quantizer.from_tq(v_quant))
 
     def get_seq_length(self, layer_idx: int = 0) -> int:
         if len(set(self.lengths)) != 1:
@@ -144,23 +145,23 @@ class PagedPackedCache:
         """Once per forward: check ownership and reservation, build the page
         table and the post-append lengths, and copy both to the device.  Never
         allocates pages: a forward racing a release must fail."""
-        refs = [self.pool.held(o) for o in self.owners]
-        for owner, held, L in zip(self.owners, refs, self.lengths):
-            if self.pool.pages_for(L + n) > len(held):
-                raise StalePage(f"{owner} holds {len(held)} pages, needs {self.pool.pages_for(L + n)}")
-            self.pool.validate(owner, held)
-        width = max(max((len(r) for r in refs), default=0), 1)
-        table = torch.full((len(refs), width), -1, dtype=torch.int32)
-        for b, held in enumerate(refs):
-            if held:
-                table[b, :len(held)] = torch.tensor([r.page for r in held], dtype=torch.int32)
-        self._refs = refs
-        self._table = table.to(device, non_blocking=True)
-        self._seq = torch.tensor([L + n for L in self.lengths], dtype=torch.int32).to(
-            device, non_blocking=True)
-        self.status = torch.zeros(1, dtype=torch.int32, device=device)
+        after = [L + n for L in self.lengths]
+        rows = self.pool.page_rows(self.owners, after)
+        B, width = len(rows), max(max((len(r) for r in rows), default=0), 1)
+        # table, lengths and the status word in one pinned buffer and one copy
+        stage = torch.empty(B * width + B + 1, dtype=torch.int32, pin_memory=device.type == "cuda")
+        words = stage.numpy()
+        words[:B * width] = -1
+        table = words[:B * width].reshape(B, width)
+        for b, held in enumerate(rows):
+            table[b, :len(held)] = held
+        words[B * width:-1] = after
+        words[-1] = 0
+        on_device = stage.to(device, non_blocking=True)
+        self._table = on_device[:B * width].view(B, width)
+        self._seq = on_device[B * width:-1]
+        self.status = on_device[-1:]
 
-    @torch.no_grad()
     def update(self, key_states, value_states, layer_idx, *args, **kwargs):
         B, Hkv, n, D = key_states.shape
         if B != len(self.owners):
@@ -170,23 +171,21 @@ class PagedPackedCache:
             self._prepare(n, dev)
         pool = self.pool
         last = layer_idx == pool.num_layers - 1
+        k_pages, k_norms, v_pages, v_norms = pool.layer(layer_idx)
         if pool.dense:
             S = pool.page_size
             pos = torch.tensor([[L + i for i in range(n)] for L in self.lengths], device=dev)
             pids = torch.gather(self._table.long(), 1, pos // S)
             slots = pos % S
-            for src, pages in ((key_states, pool.k_pages), (value_states, pool.v_pages)):
-                pages[layer_idx][pids, :, slots] = src.permute(0, 2, 1, 3).to(pages.dtype)
-            handle = pa.DenseKV(pool.k_pages[layer_idx], pool.v_pages[layer_idx],
-                                self._table, self._seq, D)
+            with torch.no_grad():
+                for src, pages in ((key_states, k_pages), (value_states, v_pages)):
+                    pages[pids, :, slots] = src.permute(0, 2, 1, 3).to(pages.dtype)
+            handle = pa.DenseKV(k_pages, v_pages, self._table, self._seq, D)
         else:
-            append_tokens(key_states, value_states, pool.k_pages[layer_idx], pool.k_norms[layer_idx],
-                          pool.v_pages[layer_idx], pool.v_norms[layer_idx], self._table, self._seq,
-                          self.kq, self.vq, status=self.status)
-            handle = pa.PackedKV(pool.k_pages[layer_idx], pool.k_norms[layer_idx],
-                                 pool.v_pages[layer_idx], pool.v_norms[layer_idx],
-                                 self._table, self._seq, pa.Quantizer.from_tq(self.kq),
-                                 pa.Quantizer.from_tq(self.vq), D)
+            append_tokens(key_states, value_states, k_pages, k_norms, v_pages, v_norms, self._table,
+                          self._seq, self.kq, self.vq, status=self.status)
+            handle = pa.PackedKV(k_pages, k_norms, v_pages, v_norms, self._table, self._seq,
+                                 *self._quants, D)
             handle.table_validated = True      # ids come from validated page refs
         handle.decode_backend = self.decode_backend
         handle.prefill_backend = self.prefill_backend
@@ -222,7 +221,6 @@ class AppendPlan:
                 or page_table.stride(-1) != 1 or not seq_lens.is_contiguous():
             raise ValueError("page_table and seq_lens must be contiguous int32")
         self.device = dev
-        self._keep = (k, v, k_pages, k_norms, v_pages, v_norms, page_table, seq_lens, k_tq, v_tq, status)
         self._sides = [
             _lib.Side(pages.data_ptr(), norms.data_ptr(), pages.stride(0), pages.stride(1),
                       norms.stride(0), norms.stride(1), tq.Pi.data_ptr(), tq.boundaries.data_ptr(),
@@ -230,6 +228,8 @@ class AppendPlan:
             for pages, norms, tq in ((k_pages, k_norms, k_tq), (v_pages, v_norms, v_tq))]
         self._ks = _lib.i64x(k.stride(0), k.stride(1), k.stride(2))
         self._vs = _lib.i64x(v.stride(0), v.stride(1), v.stride(2))
+        self._call = (k, v, k_pages, k_norms, v_pages, v_norms, page_table, seq_lens, k_tq, v_tq, order, status)
+        self._fast = _lib.host().append
         self._fn = _lib.lib().wtq_append
         self._args = (k.data_ptr(), v.data_ptr(), _lib.dtype_code(k.dtype), self._ks, self._vs,
                       ctypes.byref(self._sides[0]), ctypes.byref(self._sides[1]),
@@ -238,12 +238,13 @@ class AppendPlan:
                       status.data_ptr() if status is not None else None)
 
     def run(self) -> None:
+        if self._fast(*self._call):
+            return
         rc = self._fn(*self._args, torch.cuda.current_stream(self.device).cuda_stream)
         if rc:
             _lib.check(rc)
 
 
-@torch.no_grad()
 def append_tokens(k, v, k_pages, k_norms, v_pages, v_norms, page_table, seq_lens, k_tq, v_tq, *,
                   order: int = _lib.ORDER_AUTO, status: torch.Tensor | None = None) -> None:
     """Fused append of n tokens per sequence into one layer's pages.
@@ -253,14 +254,18 @@ def append_tokens(k, v, k_pages, k_norms, v_pages, v_norms, page_table, seq_lens
     `seq_lens` already includes the n new tokens, so token i of sequence b is
     written at position seq_lens[b] - n + i.
     """
-    if k.stride(-1) != 1:
-        k = k.contiguous()
-    if v.stride(-1) != 1:
-        v = v.contiguous()
-    plan = AppendPlan(k, v, k_pages, k_norms, v_pages, v_norms, page_table, seq_lens, k_tq, v_tq,
-                      order=order, status=status)
-    with torch.cuda.device(plan.device):
-        plan.run()
+    if _lib.host().append(k, v, k_pages, k_norms, v_pages, v_norms, page_table, seq_lens, k_tq, v_tq,
+                          order, status):
+        return
+    with torch.no_grad():
+        if k.stride(-1) != 1:
+            k = k.contiguous()
+        if v.stride(-1) != 1:
+            v = v.contiguous()
+        plan = AppendPlan(k, v, k_pages, k_norms, v_pages, v_norms, page_table, seq_lens, k_tq, v_tq,
+                          order=order, status=status)
+        with torch.cuda.device(plan.device):
+            plan.run()
 
 
 def select_decode_backend(query: torch.Tensor, kv, requested: str) -> str:
@@ -388,9 +393,12 @@ def winnow_packed_attention(module, query, key, value, attention_mask, dropout: 
         if requested == "triton_packed":
             BACKEND_COUNTS["triton_packed"] += 1
         if backend == "cuda_packed":
-            out = packed_decode_attention(
-                query, key, scaling, status=getattr(key, "status", None),
-                check_page_ids=not getattr(key, "table_validated", False))
+            status, validated = getattr(key, "status", None), getattr(key, "table_validated", False)
+            if validated:
+                out = _lib.host().attend(query, key, scaling, status)
+                if out is not None:
+                    return out, None
+            out = packed_decode_attention(query, key, scaling, status=status, check_page_ids=not validated)
         else:
             out = _reconstruct_sdpa(query, key, scaling)
     return out.transpose(1, 2).contiguous(), None

@@ -43,6 +43,9 @@ class PageRef:
     generation: int
 
 
+_NO_PAGES = np.empty(0, np.int32)
+
+
 class _Finished:
     """Fence of work that has nothing outstanding (CPU bookkeeping only)."""
 
@@ -65,13 +68,21 @@ def default_fence(device: torch.device):
 class _Reservation:
     """Pages one owner holds, in token order, with the generation each was taken at."""
 
-    __slots__ = ("slot", "pages", "generations", "version")
+    __slots__ = ("slot", "pages", "generations", "version", "_arrays")
 
     def __init__(self, slot: int):
         self.slot = slot
         self.pages: list[int] = []
         self.generations: list[int] = []
         self.version = 0                      # bumped whenever `pages` changes
+        self._arrays = (0, np.empty(0, np.int32), np.empty(0, np.int64))
+
+    def arrays(self) -> tuple[np.ndarray, np.ndarray]:
+        """`pages` and `generations` as arrays, converted once per version."""
+        if self._arrays[0] != self.version:
+            self._arrays = (self.version, np.asarray(self.pages, np.int32),
+                            np.asarray(self.generations, np.int64))
+        return self._arrays[1:]
 
     def refs(self) -> list[PageRef]:
         return [PageRef(p, g) for p, g in zip(self.pages, self.generations)]
@@ -106,6 +117,7 @@ class PagePool:
         self._retired: list[tuple[object, list[int]]] = []             # (fence, pages) per release
         self._held: dict[str, _Reservation] = {}
         self._next_slot = 0
+        self._layers = None
         self._lock = threading.Lock()
 
     # ---- accounting --------------------------------------------------------
@@ -233,17 +245,46 @@ class PagePool:
                                     f"{int(self._gen[ref.page])} and "
                                     f"{'unowned' if self._slot_of[ref.page] < 0 else 'held by another request'}")
 
+    def _check_held(self, owner: str, res: _Reservation) -> np.ndarray:
+        """`owner`'s pages in token order, every one validated (lock held)."""
+        pages, generations = res.arrays()
+        if len(pages) and (np.any(self._slot_of[pages] != res.slot)
+                           or np.any(self._gen[pages] != generations)):
+            raise StalePage(f"request {owner!r} holds a page that was released")
+        return pages
+
     def _snapshot(self, owner: str):
         """(version, pages) of `owner`'s reservation, validated as a whole."""
         with self._lock:
             res = self._held.get(owner)
             if res is None:
-                return -1, []
-            pages = np.asarray(res.pages, dtype=np.int64)
-            if len(pages) and (np.any(self._slot_of[pages] != res.slot)
-                               or np.any(self._gen[pages] != np.asarray(res.generations))):
-                raise StalePage(f"request {owner!r} holds a page that was released")
-            return res.version, list(res.pages)
+                return -1, np.empty(0, np.int32)
+            return res.version, self._check_held(owner, res)
+
+    def page_rows(self, owners, needed_tokens) -> list[np.ndarray]:
+        """The pages of every owner of a batch in token order, or `StalePage` if a
+        reservation does not cover its tokens: the rows of a forward's page table.
+        Read under the pool's lock, a reservation that is held owns its pages (they
+        leave it only with `release`, which drops the reservation), so there is
+        nothing further to validate."""
+        rows, size = [], self.page_size
+        with self._lock:
+            for owner, want in zip(owners, needed_tokens):
+                res = self._held.get(owner)
+                have = len(res.pages) if res is not None else 0
+                if want > have * size:
+                    raise StalePage(f"{owner} holds {have} pages, needs {self.pages_for(want)}")
+                rows.append(res.arrays()[0] if res is not None else _NO_PAGES)
+        return rows
+
+    def layer(self, index: int):
+        """(k_pages, k_norms, v_pages, v_norms) of one layer: views made once per
+        storage (a forward asks for them in every layer)."""
+        store = (self.k_pages, self.k_norms, self.v_pages, self.v_norms)
+        if self._layers is None or any(a is not b for a, b in zip(self._layers[0], store)):
+            views = [tuple(None if t is None else t[i] for t in store) for i in range(self.num_layers)]
+            self._layers = (store, views)
+        return self._layers[1][index]
 
 
 class DeviceTable:
@@ -279,8 +320,7 @@ class DeviceTable:
                 raise PoolExhausted(f"request {owner!r} holds {len(pages)} pages; this table is "
                                     f"{self.width} wide")
             self._stage.fill_(-1)
-            if pages:
-                self._stage[:len(pages)] = torch.as_tensor(pages, dtype=torch.int32)
+            self._stage[:len(pages)] = torch.from_numpy(pages)
             self.table[b].copy_(self._stage, non_blocking=False)
             self._seen[b] = (version, len(pages))
             changed += 1
