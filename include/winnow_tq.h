@@ -109,6 +109,10 @@ int wtq_append(const void *k, const void *v, int dtype, const int64_t k_strides[
                int Hkv, int n, int D, int S, int P, int max_pages, int order, int32_t *status,
                void *stream);
 
+/* Up to three device-to-device copies (16-byte aligned buffers, sizes in bytes, 0:
+ * none) in one launch: a decode step's K, V and query into staging buffers. */
+int wtq_stage(void *const dst[3], const void *const src[3], const int64_t bytes[3], void *stream);
+
 /* Replaces packed_decode_attention (turboquant_kv/packed_attention_triton.py:
  * 180-187, 204-262): one query token per sequence attends to its packed
  * history.  q: (B, Hq, D) of `dtype`, element strides {batch, head}; out:

@@ -53,6 +53,8 @@ _SIGNATURES = {
                            ctypes.POINTER(c_int64), ctypes.POINTER(Side), ctypes.POINTER(Side),
                            c_void_p, c_int64, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int,
                            c_int, c_int, c_void_p, c_void_p]),
+    "wtq_stage": (c_int, [ctypes.POINTER(c_void_p), ctypes.POINTER(c_void_p), ctypes.POINTER(c_int64),
+                          c_void_p]),
     "wtq_decode_workspace_bytes": (c_size_t, [c_int] * 7),
     "wtq_decode_counter_bytes": (c_size_t, [c_int, c_int]),
     "wtq_decode_auto_splits": (c_int, [c_int] * 8),

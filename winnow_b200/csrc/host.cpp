@@ -281,6 +281,39 @@ PyObject *append(PyObject *, PyObject *const *a, Py_ssize_t n) {
   Py_RETURN_TRUE;
 }
 
+// stage(dst, src, dst, src, dst, src) -> True, or None: copies of contiguous tensors of equal type and size
+// (a pair of None: nothing to copy)
+PyObject *stage(PyObject *, PyObject *const *a, Py_ssize_t n) {
+  void *dst[3] = {};
+  const void *src[3] = {};
+  int64_t bytes[3] = {};
+  at::Device dev(at::kCPU);
+  if (n != 6) Py_RETURN_NONE;
+  for (int i = 0; i < 3; ++i) {
+    if (a[2 * i + 1] == Py_None) continue;
+    at::Tensor d, s;
+    if (!tensor(a[2 * i], d) || !tensor(a[2 * i + 1], s) || !d.is_cuda() || s.device() != d.device() ||
+        d.scalar_type() != s.scalar_type() || d.sizes() != s.sizes() || !d.is_contiguous() || !s.is_contiguous() ||
+        (dev.is_cuda() && dev != d.device()))
+      Py_RETURN_NONE;
+    dev = d.device();
+    dst[i] = d.data_ptr();
+    src[i] = s.const_data_ptr();
+    bytes[i] = (int64_t)d.nbytes();
+    if ((((uintptr_t)dst[i] | (uintptr_t)src[i]) & 15) != 0) Py_RETURN_NONE;
+  }
+  if (!dev.is_cuda()) Py_RETURN_TRUE;
+  const c10::cuda::OptionalCUDAGuard guard(dev);
+  void *stream = (void *)at::cuda::getCurrentCUDAStream(dev.index()).stream();
+  int rc;
+  {
+    const Unlocked u;
+    rc = wtq_stage(dst, src, bytes, stream);
+  }
+  if (rc) return library_error(rc);
+  Py_RETURN_TRUE;
+}
+
 PyObject *set_error(PyObject *, PyObject *type) {
   Py_INCREF(type);
   Py_XSETREF(g_backend_error, type);
@@ -292,6 +325,7 @@ PyMethodDef methods[] = {
     {"attend", (PyCFunction)(void (*)(void))attend, METH_FASTCALL, "attend(q, kv, scale, status)"},
     {"append", (PyCFunction)(void (*)(void))append, METH_FASTCALL,
      "append(k, v, k_pages, k_norms, v_pages, v_norms, page_table, seq_lens, k_tq, v_tq, order, status)"},
+    {"stage", (PyCFunction)(void (*)(void))stage, METH_FASTCALL, "stage(dst, src, dst, src, dst, src)"},
     {"set_error", set_error, METH_O, "the exception type library errors are raised as"},
     {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_host", "native host side of winnow_b200", -1, methods};

@@ -20,6 +20,14 @@
 
 namespace wtq {
 
+// The rotation may be scheduled while the kernel ahead of it drains (an append, the
+// merge of the previous call).  Until the wait it reads nothing but Pi; after it,
+// every kernel ahead has completed, and only then are the scan's blocks let in, so
+// that the scan too may read pages, table and lengths before its own wait.
+__device__ __forceinline__ void begin_rotation() {
+  asm volatile("griddepcontrol.wait;\n" ::: "memory");
+}
+
 // Exclusive prefix of chunks per sequence (B + 1 ints), computed by one warp.
 __device__ void write_chunk_prefix(const int32_t *seq_lens, int B, int chunk_tokens,
                                    int max_tokens, int32_t *chunk_prefix) {
@@ -70,6 +78,7 @@ __global__ void __launch_bounds__(kRotThreads) rotate_q_kernel(
     int D, int total_rows, float *q_rot, const int32_t *seq_lens, int B, int chunk_tokens,
     int max_tokens, ScanSetup setup) {
   __shared__ float qs[NR][256];
+  begin_rotation();
   scan_setup(setup, seq_lens, B, chunk_tokens, max_tokens);
   const int row0 = blockIdx.x * NR;
   for (int e = threadIdx.x; e < NR * D; e += kRotThreads) {
@@ -372,7 +381,6 @@ __global__ void __launch_bounds__(kRotThreads) rotate_q_rows_kernel(
     int max_tokens, ScanSetup setup) {
   __shared__ __align__(16) float qs[256][NR];          // [coordinate][row]
   __shared__ float part_s[3][NR][256];
-  scan_setup(setup, seq_lens, B, chunk_tokens, max_tokens);
   const int quarter = threadIdx.x >> 7, dq = D / 4, col = threadIdx.x & 127;
   // For head_dim <= 128 a thread's share of Pi (a quarter of one row, at most 8
   // float4) stays in registers for every group of rows this block processes.
@@ -383,6 +391,8 @@ __global__ void __launch_bounds__(kRotThreads) rotate_q_rows_kernel(
 #pragma unroll
     for (int j = 0; j < 8; ++j) held[j] = (col < D && j < dq / 4) ? __ldg(row + j) : make_float4(0, 0, 0, 0);
   }
+  begin_rotation();
+  scan_setup(setup, seq_lens, B, chunk_tokens, max_tokens);
   const int groups = (total_rows + NR - 1) / NR;
   for (int grp = blockIdx.x; grp < groups; grp += gridDim.x) {
     const int row0 = grp * NR;
@@ -451,7 +461,6 @@ __global__ void __launch_bounds__(kRotThreads) rotate_q128_kernel(
     int max_tokens, ScanSetup setup) {
   __shared__ __align__(16) float qs[2][128][NR];       // [buffer][coordinate][row]
   __shared__ float part_s[3][NR][128];
-  scan_setup(setup, seq_lens, B, chunk_tokens, max_tokens);
   const int tid = threadIdx.x, col = tid & 127, quarter = tid >> 7;
   float4 held[8];                                       // this thread's quarter of row `col` of Pi
   {
@@ -459,6 +468,8 @@ __global__ void __launch_bounds__(kRotThreads) rotate_q128_kernel(
 #pragma unroll
     for (int j = 0; j < 8; ++j) held[j] = __ldg(row + j);
   }
+  begin_rotation();
+  scan_setup(setup, seq_lens, B, chunk_tokens, max_tokens);
   constexpr int PER = NR * 128 / kRotThreads;           // query elements a thread stages
   static_assert(PER >= 1, "at least four rows per group");
   float pre[PER];
@@ -526,34 +537,36 @@ int launch_rotate_q(const void *q, int dtype, const int64_t *qs, const float *Pi
                     int B, int Hq, int D, float *q_rot, const int32_t *seq_lens, int chunk_tokens,
                     int max_tokens, const ScanSetup &setup, cudaStream_t stream) {
   const int rows = B * Hq;
+  const bool pi_words = ((uintptr_t)Pi & 15) == 0;
+  cudaLaunchAttribute pdl;
+  pdl.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  pdl.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.blockDim = dim3(kRotThreads);
+  cfg.stream = stream;
+  cfg.attrs = &pdl;
+  cfg.numAttrs = 1;
+  cudaError_t e;
+  auto fixed = [&](auto kernel, int nr, int most) {            // head_dim 128
+    cfg.gridDim = dim3((unsigned)std::min((rows + nr - 1) / nr, most));
+    e = cudaLaunchKernelEx(&cfg, kernel, q, dtype, qs[0], qs[1], Pi, scale, Hq, rows, q_rot, seq_lens, B,
+                           chunk_tokens, max_tokens, setup);
+  };
+  auto general = [&](auto kernel, int nr, int most) {
+    cfg.gridDim = dim3((unsigned)std::min((rows + nr - 1) / nr, most));
+    e = cudaLaunchKernelEx(&cfg, kernel, q, dtype, qs[0], qs[1], Pi, scale, Hq, D, rows, q_rot, seq_lens, B,
+                           chunk_tokens, max_tokens, setup);
+  };
   // (two 512-thread blocks of the head_dim-128 kernel fit an SM, one of the general kernel)
-  if (D == 128 && ((uintptr_t)Pi & 15) == 0 && rows >= 8 * 148)
-    rotate_q128_kernel<8><<<std::min((rows + 7) / 8, 2 * 148), kRotThreads, 0, stream>>>(
-        q, dtype, qs[0], qs[1], Pi, scale, Hq, rows, q_rot, seq_lens, B, chunk_tokens, max_tokens,
-        setup);
-  else if (D == 128 && ((uintptr_t)Pi & 15) == 0)
-    rotate_q128_kernel<4><<<std::min((rows + 3) / 4, 2 * 148), kRotThreads, 0, stream>>>(
-        q, dtype, qs[0], qs[1], Pi, scale, Hq, rows, q_rot, seq_lens, B, chunk_tokens, max_tokens,
-        setup);
-  else if (D % 16 == 0 && D <= 256 && ((uintptr_t)Pi & 15) == 0 && rows >= 8 * 148)
-    // many rows: eight per pass halve the passes of the persistent blocks
-    rotate_q_rows_kernel<8><<<std::min((rows + 7) / 8, 148), kRotThreads, 0, stream>>>(
-        q, dtype, qs[0], qs[1], Pi, scale, Hq, D, rows, q_rot, seq_lens, B, chunk_tokens,
-        max_tokens, setup);
-  else if (D % 16 == 0 && D <= 256 && ((uintptr_t)Pi & 15) == 0)
-    rotate_q_rows_kernel<4><<<std::min((rows + 3) / 4, 148), kRotThreads, 0, stream>>>(
-        q, dtype, qs[0], qs[1], Pi, scale, Hq, D, rows, q_rot, seq_lens, B, chunk_tokens,
-        max_tokens, setup);
-  else if (rows % 4 == 0)
-    rotate_q_kernel<4><<<rows / 4, kRotThreads, 0, stream>>>(
-        q, dtype, qs[0], qs[1], Pi, scale, Hq, D, rows, q_rot, seq_lens, B, chunk_tokens,
-        max_tokens, setup);
-  else
-    rotate_q_kernel<1><<<rows, kRotThreads, 0, stream>>>(
-        q, dtype, qs[0], qs[1], Pi, scale, Hq, D, rows, q_rot, seq_lens, B, chunk_tokens,
-        max_tokens, setup);
+  if (D == 128 && pi_words && rows >= 8 * 148) fixed(rotate_q128_kernel<8>, 8, 2 * 148);
+  else if (D == 128 && pi_words) fixed(rotate_q128_kernel<4>, 4, 2 * 148);
+  // many rows: eight per pass halve the passes of the persistent blocks
+  else if (D % 16 == 0 && D <= 256 && pi_words && rows >= 8 * 148) general(rotate_q_rows_kernel<8>, 8, 148);
+  else if (D % 16 == 0 && D <= 256 && pi_words) general(rotate_q_rows_kernel<4>, 4, 148);
+  else if (rows % 4 == 0) general(rotate_q_kernel<4>, 4, 1 << 30);
+  else general(rotate_q_kernel<1>, 1, 1 << 30);
   note_launches(1);
-  return check_cuda(cudaGetLastError(), "wtq_decode rotate launch");
+  return check_cuda(e, "wtq_decode rotate launch");
 }
 
 int launch_merge(const MergeParams &p, int B, cudaStream_t stream) {

@@ -232,3 +232,58 @@ extern "C" int wtq_unpack(const uint8_t *packed, uint8_t *idx, int64_t rows, int
   note_launches(1);
   return check_cuda(cudaGetLastError(), "wtq_unpack launch");
 }
+
+// ---- staging -------------------------------------------------------------------
+// Up to three device-to-device copies in one launch: the key, value and query of a
+// decode step's layer on their way into fixed staging buffers (three copy launches
+// cost more than the bytes do).
+namespace {
+struct StageJob {
+  void *dst[3];
+  const void *src[3];
+  int64_t bytes[3];
+};
+__global__ void __launch_bounds__(256) stage_kernel(StageJob job) {
+  asm volatile("griddepcontrol.wait;\n" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+  const int64_t first = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, step = (int64_t)gridDim.x * blockDim.x;
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    const int64_t n16 = job.bytes[i] >> 4;
+    const uint4 *src = (const uint4 *)job.src[i];
+    uint4 *dst = (uint4 *)job.dst[i];
+    for (int64_t e = first; e < n16; e += step) dst[e] = src[e];
+    const int64_t tail = (n16 << 4) + first;
+    if (tail < job.bytes[i]) ((uint8_t *)job.dst[i])[tail] = ((const uint8_t *)job.src[i])[tail];
+  }
+}
+}  // namespace
+
+extern "C" int wtq_stage(void *const dst[3], const void *const src[3], const int64_t bytes[3],
+                         void *stream) {
+  if (!dst || !src || !bytes) return fail(WTQ_ERR_ARG, "wtq_stage: null descriptor");
+  StageJob job;
+  int64_t most = 0;
+  for (int i = 0; i < 3; ++i) {
+    if (bytes[i] < 0 || (bytes[i] > 0 && (!dst[i] || !src[i])))
+      return fail(WTQ_ERR_ARG, "wtq_stage: null buffer or negative size");
+    if (bytes[i] > 0 && (((uintptr_t)dst[i] | (uintptr_t)src[i]) & 15))
+      return fail(WTQ_ERR_UNSUPPORTED, "wtq_stage: buffers must be 16-byte aligned");
+    job.dst[i] = dst[i]; job.src[i] = src[i]; job.bytes[i] = bytes[i];
+    most = bytes[i] > most ? bytes[i] : most;
+  }
+  if (most == 0) return WTQ_OK;
+  const int64_t blocks = (most / 16 + 255) / 256;
+  cudaLaunchAttribute pdl;
+  pdl.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  pdl.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(blocks < 1 ? 1 : blocks > 8 * device_sms() ? 8 * device_sms() : blocks));
+  cfg.blockDim = dim3(256);
+  cfg.stream = (cudaStream_t)stream;
+  cfg.attrs = &pdl;
+  cfg.numAttrs = 1;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, stage_kernel, job);
+  note_launches(1);
+  return check_cuda(e, "wtq_stage launch");
+}

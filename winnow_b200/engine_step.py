@@ -72,6 +72,7 @@ class DecodeSession:
                                            out=self.out, workspace=ws, status=self.status,
                                            check_page_ids=False))
         self._graphs = None
+        self._host = _lib.host()
         self._one = torch.ones((), dtype=torch.int32, device=dev)
 
     # ---- step protocol -----------------------------------------------------------
@@ -91,12 +92,10 @@ class DecodeSession:
         """Append the new token's K/V of this layer and attend; returns `out`
         (overwritten by the next layer).  k, v: (B, Hkv, 1, D); q: (B, Hq, 1, D);
         omitted ones are taken from the staging tensors as they are."""
-        if k is not None:
-            self.k_in.copy_(k)
-        if v is not None:
-            self.v_in.copy_(v)
-        if q is not None:
-            self.q_in.copy_(q)
+        if not self._host.stage(self.k_in, k, self.v_in, v, self.q_in, q):   # one launch, else copy by copy
+            for into, given in ((self.k_in, k), (self.v_in, v), (self.q_in, q)):
+                if given is not None:
+                    into.copy_(given)
         if self._graphs is not None:
             self._graphs[layer_idx].replay()
         else:
