@@ -265,12 +265,27 @@ class TQPackedLayer(_LayerBase):
             self._mask = mask
             self._channels = ((~mask).nonzero().flatten(), mask.nonzero().flatten())
         self._shape = (B, H, D)
+        self._ring_table = torch.arange(B, dtype=torch.int32, device=dev)[:, None]
+        self._ring_len = torch.zeros(B, dtype=torch.int32, device=dev)
         self.last_dispatch_decision = (self._dispatcher or default_dispatcher()).select(
             Hardware.from_torch(torch, dev), Shape(B, H, self._max, D, self._bw),
             NumericalContract.quantization_aware())
         if self.last_dispatch_decision.backend == "none":
             raise _lib.BackendError(self.last_dispatch_decision.reason)
         self.is_initialized = True
+
+    def _store_both(self, ks, vs, pos, n) -> bool:
+        """K and V of n new tokens into the rings with one fused append (the rings are
+        pages of `max_cache_len` tokens, one per sequence); False where outlier
+        channels or the source type need the part-by-part form."""
+        if self._out_dim or ks.dtype != vs.dtype or ks.dtype not in (torch.float32, torch.float16,
+                                                                     torch.bfloat16):
+            return False
+        from .packed_backend import append_tokens
+        self._ring_len.fill_(pos + n)
+        append_tokens(ks, vs, self._k[0], self._k[1], self._v[0], self._v[1], self._ring_table,
+                      self._ring_len, self._tq, self._tq)
+        return True
 
     def _store(self, x, pos, n, side):
         parts = ((self._tq, None, 0),) if not self._out_dim else (
@@ -304,8 +319,9 @@ class TQPackedLayer(_LayerBase):
         if self._len + n > self._max:
             raise RuntimeError(f"TQPackedLayer overflow: {self._len}+{n} > max_cache_len="
                                f"{self._max}. Raise max_cache_len.")
-        self._store(key_states, self._len, n, self._k)
-        self._store(value_states, self._len, n, self._v)
+        if not n or not self._store_both(key_states, value_states, self._len, n):
+            self._store(key_states, self._len, n, self._k)
+            self._store(value_states, self._len, n, self._v)
         self._len += n
         return self._load(self._len, self._k), self._load(self._len, self._v)
 

@@ -17,6 +17,8 @@
 //              (s0+s1)+(s2+s3);
 //   bucket   : number of boundaries strictly below y (bucketize, right=False);
 //   norm out : fp16 round-to-nearest-even for pages, fp32 for wtq_quantize.
+#include <atomic>
+
 #include "wtq_quant.cuh"
 
 namespace wtq {
@@ -255,6 +257,169 @@ __global__ void append_kernel(AppendParams p) {
   }
 }
 
+// A decode step's append at head_dim 128: NV vectors per block, one coordinate per
+// thread.  Few vectors leave no arithmetic to save: the step takes as long as its
+// dependent pieces (where the token goes, norm, division, one chain of 128 FMAs,
+// bucket), so here every coordinate runs its chain (wtq_quant_mma.cu runs them only
+// near boundaries, and has more phases).  Pi comes into shared memory with coalesced
+// copies issued before griddepcontrol.wait, under the tail of the kernel ahead;
+// reading it row by row from global memory cost every block 128 x 32 sectors a warp.
+// 32 / 128 / 256 / 512 vectors a side: 6.6 / 6.8 / 7.3 / 8.9 us (before 10.7 to 11.1);
+// 1024 would take 17.4, the tensor-core kernel 13.8.
+constexpr int kFewVectors = 512;                             // per side
+constexpr int kPiRow = 132;                                  // floats per row: conflict-free 16-byte reads
+template <int NV> struct FewSmem {
+  float pi[128][kPiRow];
+  float x[NV][128];
+  float lane[NV][8];
+  float norm[NV];
+  float bounds[255];
+  uint8_t idx[NV][128];
+  int64_t dest[NV][2];
+};
+template <int NV>
+__global__ void __launch_bounds__(128) append_few_kernel(AppendParams p) {
+  extern __shared__ __align__(16) uint8_t smem_raw[];
+  FewSmem<NV> &s = *reinterpret_cast<FewSmem<NV> *>(smem_raw);
+  const AppendSideDev &a = p.side[blockIdx.y];
+  const int c = threadIdx.x;
+#pragma unroll 8
+  for (int e = c; e < 128 * 32; e += 128) {
+    const uint32_t dst = (uint32_t)__cvta_generic_to_shared(&s.pi[e >> 5][4 * (e & 31)]);
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst), "l"(a.q.Pi + 4 * e) : "memory");
+  }
+  asm volatile("cp.async.commit_group;\n" ::: "memory");
+  for (int e = c; e < a.q.nbounds; e += 128) s.bounds[e] = a.q.bounds[e];
+  asm volatile("griddepcontrol.wait;\n" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+  const int64_t vectors = (int64_t)p.B * p.Hkv * p.n, v0 = (int64_t)blockIdx.x * NV;
+  if (c < NV) {
+    // Where the token goes; -1 marks a position or page the table does not
+    // cover (reported through `status`, not written) or a vector past the end.
+    const int64_t vec = v0 + c;
+    int64_t code_off = -1, norm_off = -1;
+    if (vec < vectors) {
+      const int i = (int)(vec % p.n);
+      const int h = (int)((vec / p.n) % p.Hkv);
+      const int b = (int)(vec / ((int64_t)p.n * p.Hkv));
+      const int pos = p.seq_lens[b] - p.n + i;
+      const int slot_page = pos >= 0 ? pos / p.S : -1;
+      if (pos < 0 || slot_page >= p.max_pages) {
+        if (p.status) atomicOr(p.status, WTQ_STATUS_BAD_POSITION);
+      } else {
+        const int pid = p.page_table[(int64_t)b * p.table_stride + slot_page];
+        if (pid < 0 || pid >= p.P) {
+          if (p.status) atomicOr(p.status, WTQ_STATUS_BAD_PAGE);
+        } else {
+          const int slot = pos - slot_page * p.S;
+          code_off = (int64_t)pid * a.page_stride + (int64_t)h * a.head_stride + (int64_t)slot * a.q.nb;
+          norm_off = (int64_t)pid * a.norm_page_stride + (int64_t)h * a.norm_head_stride + slot;
+        }
+      }
+    }
+    s.dest[c][0] = code_off;
+    s.dest[c][1] = norm_off;
+  }
+#pragma unroll
+  for (int j = 0; j < NV; ++j) {
+    const int64_t vec = v0 + j;
+    float v = 0.0f;
+    if (vec < vectors) {
+      const int i = (int)(vec % p.n);
+      const int h = (int)((vec / p.n) % p.Hkv);
+      const int b = (int)(vec / ((int64_t)p.n * p.Hkv));
+      v = load_as_float(a.src, (int64_t)b * a.sb + (int64_t)h * a.sh + (int64_t)i * a.st + c, p.dtype);
+    }
+    s.x[j][c] = v;
+  }
+  __syncthreads();
+  if (c < 8 * NV) {
+    const int j = c >> 3, l = c & 7;
+    float acc = 0.0f;
+#pragma unroll
+    for (int d = l; d < 128; d += 8) acc = __fadd_rn(acc, __fmul_rn(s.x[j][d], s.x[j][d]));
+    s.lane[j][l] = acc;
+  }
+  __syncthreads();
+  // every thread adds the eight partial sums itself: no further barrier before the division
+  float norm[NV];
+#pragma unroll
+  for (int j = 0; j < NV; ++j) {
+    float t = s.lane[j][0];
+#pragma unroll
+    for (int l = 1; l < 8; ++l) t = __fadd_rn(t, s.lane[j][l]);
+    norm[j] = fmaxf(__fsqrt_rn(t), 1e-10f);
+    s.x[j][c] = __fdiv_rn(s.x[j][c], norm[j]);
+  }
+  asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+  __syncthreads();
+  float acc[NV];
+#pragma unroll
+  for (int j = 0; j < NV; ++j) acc[j] = 0.0f;
+#pragma unroll 8
+  for (int k = 0; k < 32; ++k) {
+    const float4 w = *reinterpret_cast<const float4 *>(&s.pi[c][4 * k]);
+#pragma unroll
+    for (int j = 0; j < NV; ++j) {
+      const float4 x = *reinterpret_cast<const float4 *>(&s.x[j][4 * k]);
+      acc[j] = __fmaf_rn(x.x, w.x, acc[j]);
+      acc[j] = __fmaf_rn(x.y, w.y, acc[j]);
+      acc[j] = __fmaf_rn(x.z, w.z, acc[j]);
+      acc[j] = __fmaf_rn(x.w, w.w, acc[j]);
+    }
+  }
+  int lo[NV], hi[NV];
+#pragma unroll
+  for (int j = 0; j < NV; ++j) {
+    lo[j] = 0;
+    hi[j] = a.q.nbounds;
+  }
+  for (int step = 0; step < a.q.bw; ++step) {                // 2^bw - 1 boundaries: bw halvings
+#pragma unroll
+    for (int j = 0; j < NV; ++j) {
+      const int mid = (lo[j] + hi[j]) >> 1;
+      if (s.bounds[mid] < acc[j]) lo[j] = mid + 1;
+      else hi[j] = mid;
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < NV; ++j) s.idx[j][c] = (uint8_t)lo[j];
+  __syncthreads();
+#pragma unroll
+  for (int j = 0; j < NV; ++j) {
+    if (s.dest[j][0] >= 0) {
+      if (c < a.q.nb) a.pages[s.dest[j][0] + c] = packed_byte(s.idx[j], c, a.q.bw);
+      if (c == 0) a.norms[s.dest[j][1]] = __float2half_rn(norm[j]);
+    }
+  }
+}
+
+static int launch_append_few(const AppendParams &p, int64_t vectors, cudaStream_t stream) {
+  constexpr int NV = 4;
+  static std::atomic<bool> opted_in_dev[64];
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev >= 64 || !opted_in_dev[dev & 63].load(std::memory_order_acquire)) {
+    const cudaError_t e = cudaFuncSetAttribute(append_few_kernel<NV>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               (int)sizeof(FewSmem<NV>));
+    if (e != cudaSuccess) return check_cuda(e, "wtq_append: set-up");
+    opted_in_dev[dev & 63].store(true, std::memory_order_release);
+  }
+  cudaLaunchAttribute pdl;
+  pdl.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  pdl.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)((vectors + NV - 1) / NV), 2);
+  cfg.blockDim = dim3(128);
+  cfg.dynamicSmemBytes = sizeof(FewSmem<NV>);
+  cfg.stream = stream;
+  cfg.attrs = &pdl;
+  cfg.numAttrs = 1;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, append_few_kernel<NV>, p);
+  note_launches(1);
+  return check_cuda(e, "wtq_append launch");
+}
+
 static int block_threads(int D) { return ((D + 31) / 32) * 32; }
 
 template <typename K, typename P>
@@ -366,7 +531,9 @@ extern "C" int wtq_append(const void *k, const void *v, int dtype, const int64_t
   job.vectors = vectors; job.dtype = dtype; job.page_table = page_table; job.table_stride = table_stride;
   job.seq_lens = seq_lens; job.Hkv = Hkv; job.n = n; job.S = S; job.P = P; job.max_pages = max_pages;
   job.status = status;
-  if (quant_mma_eligible(D, p.order, job, 2))
+  const bool tensor = quant_mma_eligible(D, p.order, job, 2);
+  if (tensor && vectors <= kFewVectors) return launch_append_few(p, vectors, (cudaStream_t)stream);
+  if (tensor)
     return launch_quant_mma(job, true, 2, (cudaStream_t)stream, "wtq_append launch");
   return launch_staged(append_kernel<true>, append_kernel<false>, p, D, vectors, 2,
                        (cudaStream_t)stream, "wtq_append launch");

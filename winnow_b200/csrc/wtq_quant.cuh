@@ -35,9 +35,10 @@ struct QuantJob {
   const int32_t *seq_lens;
   int Hkv, n, S, P, max_pages;
   int32_t *status;
+  int team_shift;             // set by launch_quant_mma
 };
 
 bool quant_mma_eligible(int D, int order, const QuantJob &job, int sides);
-int launch_quant_mma(const QuantJob &job, bool append, int sides, cudaStream_t stream, const char *what);
+int launch_quant_mma(QuantJob job, bool append, int sides, cudaStream_t stream, const char *what);
 
 }  // namespace wtq
