@@ -3,38 +3,42 @@
 // page read and decoded once for all the query rows that share it.  Replaces
 // the reference's prefill fallback, which dequantizes the whole history of
 // each sequence to the model dtype and calls SDPA
-// (turboquant_kv/packed_backend.py:192-226), and this library's own earlier
-// form of it (B * Q one-token rows through the decode kernels, the history
-// read Q times).
+// (turboquant_kv/packed_backend.py:192-226).
 //
-// Work is cut into items (sequence b, kv head, block of 256 query rows, chunk
+// Work is cut into items (sequence b, kv head, block of 256 query rows, range
 // of the history); the query rows of a kv head are (token i, head r) pairs in
-// token-major order, so the causal length never decreases along them.  A block
-// of eight warps takes items from a counter.  Per item it loads its 256 rotated
-// query rows as fp16 into shared memory once, then walks the chunk in tiles of
-// 64 tokens:
+// token-major order, so the causal length never decreases along them.  Per item
+// the 256 rotated query rows go to shared memory as fp16 once, as two M = 128
+// operands; the range is then walked in tiles of 64 tokens by three groups of
+// warps that meet only at mbarriers:
 //
-//   copy     cp.async brings the tile's packed K and V rows and their fp16 norms
-//            into a landing buffer, one tile ahead of the arithmetic;
-//   decode   each warp turns one 16-token group of one side into fp16 centroid
-//            values through the per-lane lookup tables (wtq_lut.cuh) and stores
-//            them as a [token][coordinate] tile, 16-byte pieces XOR-swizzled by
-//            the row so that ldmatrix reads it without bank conflicts;
-//   scores   each warp owns 32 query rows: S = Q K^T with mma.m16n8k16 (A: query
-//            fragments by ldmatrix, B: key tile by ldmatrix; the tile holds
-//            centroid x norm), causal mask where the tile reaches a row's limit;
-//   softmax  online, in the exp2 domain, on the score fragments in registers;
-//   values   O += P V (V tile = centroid x norm), the probability fragments
-//            feeding the MMA as A operands directly, V by ldmatrix.trans.
+//   decode    seven warps: tasks of 16 tokens of one side (K or V), from packed codes
+//             loaded into registers a task ahead to fp16 centroid x norm
+//             through the per-lane lookup tables (wtq_lut.cuh) and stores them in
+//             the canonical no-swizzle operand layout, two tiles deep;
+//   multiply  one thread issues tcgen05.mma: S = Q K^T (N 64, K-major operands) one
+//             tile ahead of O += P V (A = P from tensor memory, B = V with the
+//             coordinates contiguous, i.e. MN-major: the same bytes as a K tile
+//             read with the two strides exchanged);
+//   softmax   two warpgroups, one per M tile, a thread per query row: scores from
+//             tensor memory, causal mask, online softmax in the exp2 domain, the
+//             probabilities back to tensor memory as fp16 over the scores they came
+//             from.  The reference maximum is raised, and O rescaled, only when a
+//             row's scores exceed it by 2^8, so almost no tile touches O.
 //
-// fp16 scores are exact enough while they are small; a warp whose tile holds a
-// score beyond 8 (log2 domain) recomputes that tile's scores in fp32 from the
-// packed codes.  At the end of the chunk every row that sees the chunk writes
-// its state (reference maximum, sum, un-normalised accumulator in the value
-// basis) in the layout of the decode scan, and the decode path's merge kernels
-// combine the chunks, rotate back and store.
+// Tensor memory: S of two M tiles x two buffers x 64 columns, O of two M tiles x 128.
+// fp16 scores are exact enough while they are small; a warp whose tile holds a row
+// maximum beyond 8 (log2 domain) recomputes that tile's scores in fp32 from the
+// packed codes.  At the end of the range every row that sees it writes its state
+// (reference maximum, sum, un-normalised accumulator in the value basis) in the
+// layout of the decode scan; a merge kernel combines the ranges, rotates back and
+// stores.  (The mma.sync form of this kernel, a warp per 32 rows decoding and multiplying
+// in turn, took 518 us for 137 GFLOP: its accumulators and scores filled the register
+// file and left two warps a scheduler to hide every latency.)  Every wait is bounded; one that runs out raises a flag that ends all the
+// others, and the status word says so.
 #include <algorithm>
 #include <atomic>
+#include <type_traits>
 
 #include "wtq_decode.cuh"
 #include "wtq_lut.cuh"
@@ -42,21 +46,36 @@
 namespace wtq {
 namespace pf {
 
-constexpr int kWarps = 8, kThreads = 32 * kWarps;
-constexpr int kRows = 32 * kWarps;              // query rows per item
+constexpr int kSoftWarps = 8, kDecodeWarps = 7, kMmaWarp = kSoftWarps + kDecodeWarps;   // 16 warps of 128 registers
+constexpr int kThreads = 32 * (kMmaWarp + 1);
+constexpr int kRows = 256;                      // query rows per item: two M = 128 operands
 constexpr int kTile = 64;                       // tokens per tile
 constexpr uint32_t kBase = 1024;                // dynamic shared memory is assumed to start at or below this
-constexpr uint32_t kKTile = kBase;              // [64][128] fp16
-constexpr uint32_t kVTile = kKTile + kTile * 256;
-constexpr uint32_t kNormK = kVTile + kTile * 256;   // 64 floats each
-constexpr uint32_t kNormV = kNormK + kTile * 4;
-constexpr uint32_t kItem = kNormV + kTile * 4;      // the item being worked on (8 words)
+// mbarriers (8 bytes each).  All that can be up to two tiles apart exist per buffer, so
+// that no side is ever two completions ahead of a phase another side still waits for.
+constexpr uint32_t kKFull = kBase, kVFull = kBase + 16, kKFree = kBase + 32, kVFree = kBase + 48;   // [buffer]
+constexpr uint32_t kSFull = kBase + 64;             // [M tile][buffer]: scores are in tensor memory
+constexpr uint32_t kPFull = kBase + 96;             // [M tile][buffer]: probabilities are in tensor memory
+constexpr uint32_t kODone = kBase + 128;            // [M tile][buffer]: the products of a tile into O are complete
+constexpr uint32_t kTmemSlot = kBase + 160;         // tensor-memory address written by tcgen05.alloc
+constexpr uint32_t kAbort = kBase + 164;            // a wait ran out
+constexpr uint32_t kItem = kBase + 176;             // the item being worked on (8 words)
 constexpr uint32_t kWalk = kItem + 32;              // balanced schedule: where this block stands (10 words)
-constexpr uint32_t kPlan = kWalk + 64;              // balanced schedule: tiles of every (sequence, row block)
+constexpr uint32_t kTileBytes = kTile * 256;        // a decoded tile: [64 tokens][128] fp16
+constexpr uint32_t kVTile = 2048;                   // two buffers
+constexpr uint32_t kPlan = kVTile + 2 * kTileBytes; // balanced schedule: tiles of every (sequence, row block)
 constexpr int kMaxPairs = 4096;                     // (sequence, row block) pairs the plan has room for
 constexpr int kBalancedSlots = 3;                   // a group is cut by at most two block boundaries
-static_assert(kPlan + 4 * kMaxPairs <= mma::kLutAddr, "tiles and the plan must end below the lookup tables");
+static_assert(kWalk + 64 <= kVTile && kPlan + 4 * kMaxPairs <= mma::kLutAddr, "low region");
 constexpr float kPreciseAbove = 8.f;            // |score| (log2 domain) beyond which fp16 is not trusted
+constexpr float kSlack = 8.f;                   // how far scores may exceed the reference before it is raised
+// tensor memory columns
+constexpr uint32_t kColS = 0;                   // + 128 * (M tile) + 64 * buffer; P over the first 32 of each
+constexpr uint32_t kColO = 256;                 // + 128 * (M tile)
+constexpr uint32_t kCols = 512;
+// instruction descriptors: dense, fp32 accumulator, fp16 A and B, M = 128
+constexpr uint32_t kIdescQK = (1u << 4) | ((64u >> 3) << 17) | ((128u >> 4) << 24);
+constexpr uint32_t kIdescPV = (1u << 4) | (1u << 16) | ((128u >> 3) << 17) | ((128u >> 4) << 24);   // B MN-major
 
 struct Params {
   DecodeSideDev k, v;
@@ -74,56 +93,114 @@ struct Params {
 };
 
 template <int BWK, int BWV> struct Map {
-  static constexpr int kNBK = 16 * BWK, kNBV = 16 * BWV;
   static constexpr uint32_t kLutBytes =
       (uint32_t)(mma::lut_entries(BWK) > mma::lut_entries(BWV) ? mma::lut_entries(BWK)
                                                                 : mma::lut_entries(BWV)) * 256u;
   static constexpr uint32_t kQTile = mma::kLutAddr + kLutBytes;        // [256][128] fp16
-  static constexpr uint32_t kRaw = kQTile + kRows * 256;
-  // landing buffer of one tile: K rows, V rows, K norms, V norms
-  static constexpr uint32_t kRawV = kTile * kNBK;
-  static constexpr uint32_t kRawNK = kRawV + kTile * kNBV;
-  static constexpr uint32_t kRawNV = kRawNK + kTile * 2;
-  static constexpr uint32_t kRawBytes = kRawNV + kTile * 2;
-  static constexpr uint32_t kDynamic = kRaw + 2 * kRawBytes;
+  static constexpr uint32_t kKTile = kQTile + kRows * 256;             // two buffers
+  static constexpr uint32_t kDynamic = kKTile + 2 * kTileBytes;
   static_assert(kDynamic <= 227u * 1024u, "shared memory budget");
 };
 
-__device__ __forceinline__ void ldmatrix_x4(uint32_t a, uint32_t (&r)[4]) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];\n"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(a));
-}
-__device__ __forceinline__ void ldmatrix_x4_trans(uint32_t a, uint32_t (&r)[4]) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];\n"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(a));
-}
 __device__ __forceinline__ void sts128(uint32_t a, uint32_t x, uint32_t y, uint32_t z, uint32_t w) {
   asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};\n" ::"r"(a), "r"(x), "r"(y), "r"(z), "r"(w)
                : "memory");
 }
-__device__ __forceinline__ void sts64u(uint32_t a, uint32_t x, uint32_t y) {
-  asm volatile("st.shared.v2.u32 [%0], {%1,%2};\n" ::"r"(a), "r"(x), "r"(y) : "memory");
+// ---- operand layout: core matrices of 8 rows x 16 bytes (128 bytes each); the 16 pieces
+// of a group of eight rows follow one another (2 KB per group) --------------------------
+__device__ __forceinline__ uint32_t operand_at(uint32_t tile, int row, int piece) {
+  return tile + (uint32_t)(row >> 3) * 2048u + (uint32_t)piece * 128u + (uint32_t)(row & 7) * 16u;
 }
-__device__ __forceinline__ float2 lds_f2(uint32_t a) {
-  float2 v;
-  asm volatile("ld.shared.v2.f32 {%0,%1}, [%2];\n" : "=f"(v.x), "=f"(v.y) : "r"(a));
-  return v;
+__device__ __forceinline__ uint64_t descriptor(uint32_t start, uint32_t leading, uint32_t stride) {
+  return (uint64_t)((start >> 4) & 0x3fffu) | ((uint64_t)(leading >> 4) << 16) |
+         ((uint64_t)(stride >> 4) << 32) | ((uint64_t)1 << 46);          // version, no swizzle
 }
-// 16 bytes global -> shared; `bytes` = 16, or 0 to fill the piece with zeros
-__device__ __forceinline__ void copy16(uint32_t dst, const void *src, int bytes) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst), "l"(src), "r"(bytes)
-               : "memory");
+// K-major operand (rows = M or N, contraction along a row): step ks takes pieces 2 ks, 2 ks + 1;
+// leading offset: next piece, stride offset: next eight rows
+__device__ __forceinline__ uint64_t desc_k_major(uint32_t tile, int ks) {
+  return descriptor(tile + (uint32_t)ks * 256u, 128u, 2048u);
 }
-
-// Address of 16-byte piece `piece` (0..15) of row `row` in a [rows][128] fp16 tile.
-__device__ __forceinline__ uint32_t tile_at(uint32_t tile, int row, int piece) {
-  return tile + (uint32_t)row * 256u + (uint32_t)((piece ^ (row & 7)) << 4);
+// MN-major operand (rows = contraction): step ks takes rows 16 ks .. 16 ks + 15; leading
+// offset: next eight rows, stride offset: next piece
+__device__ __forceinline__ uint64_t desc_mn_major(uint32_t tile, int ks) {
+  return descriptor(tile + (uint32_t)ks * 4096u, 2048u, 128u);
 }
+__device__ __forceinline__ void umma_ss(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %5, %5, %5}, p;\n\t}\n"
+      ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"(accumulate), "r"(0u) : "memory");
+}
+__device__ __forceinline__ void umma_ts(uint32_t d, uint32_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, {%5, %5, %5, %5}, p;\n\t}\n"
+      ::"r"(d), "r"(a), "l"(b), "r"(idesc), "r"(accumulate), "r"(0u) : "memory");
+}
+__device__ __forceinline__ void umma_commit(uint32_t bar) {
+  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ void fence_before() { asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory"); }
+__device__ __forceinline__ void fence_after() { asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory"); }
+__device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
+  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(bar), "r"(count) : "memory");
+}
+__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(bar) : "memory");
+}
+// Bounded wait for completion number `use` (0, 1, ..) of an mbarrier; false if it, or any
+// other wait of the block, ran out.
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, int use) {
+  for (int spin = 0; spin < (1 << 20); ++spin) {
+    uint32_t done;
+    asm volatile(
+        "{\n\t.reg .pred q;\n\tmbarrier.try_wait.parity.shared::cta.b64 q, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, q;\n\t}\n"
+        : "=r"(done) : "r"(bar), "r"((uint32_t)(use & 1)) : "memory");
+    if (done) return true;
+    if ((spin & 255) == 255 && lds32(kAbort) != 0u) return false;
+  }
+  sts32(kAbort, 0x80000000u | (threadIdx.x >> 5) << 24 | ((uint32_t)use & 0xfffu) << 12 | (bar - kBase));   // who gave up on what
+  return false;
+}
+template <int AT, int N> __device__ __forceinline__ void tmem_load32(uint32_t addr, uint32_t (&r)[N]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
+      "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];\n"
+      : "=r"(r[AT + 0]), "=r"(r[AT + 1]), "=r"(r[AT + 2]), "=r"(r[AT + 3]),
+        "=r"(r[AT + 4]), "=r"(r[AT + 5]), "=r"(r[AT + 6]), "=r"(r[AT + 7]),
+        "=r"(r[AT + 8]), "=r"(r[AT + 9]), "=r"(r[AT + 10]), "=r"(r[AT + 11]),
+        "=r"(r[AT + 12]), "=r"(r[AT + 13]), "=r"(r[AT + 14]), "=r"(r[AT + 15]),
+        "=r"(r[AT + 16]), "=r"(r[AT + 17]), "=r"(r[AT + 18]), "=r"(r[AT + 19]),
+        "=r"(r[AT + 20]), "=r"(r[AT + 21]), "=r"(r[AT + 22]), "=r"(r[AT + 23]),
+        "=r"(r[AT + 24]), "=r"(r[AT + 25]), "=r"(r[AT + 26]), "=r"(r[AT + 27]),
+        "=r"(r[AT + 28]), "=r"(r[AT + 29]), "=r"(r[AT + 30]), "=r"(r[AT + 31])
+      : "r"(addr));
+}
+__device__ __forceinline__ void tmem_store32(uint32_t addr, const uint32_t (&v)[32]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%32], {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
+      "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31};\n"
+      ::"r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]),
+        "r"(v[8]), "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]),
+        "r"(v[16]), "r"(v[17]), "r"(v[18]), "r"(v[19]), "r"(v[20]), "r"(v[21]), "r"(v[22]), "r"(v[23]),
+        "r"(v[24]), "r"(v[25]), "r"(v[26]), "r"(v[27]), "r"(v[28]), "r"(v[29]), "r"(v[30]), "r"(v[31]), "r"(addr)
+      : "memory");
+}
+__device__ __forceinline__ void tmem_store16(uint32_t addr, const uint32_t (&v)[16]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%16], {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15};\n"
+      ::"r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]),
+        "r"(v[8]), "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]), "r"(addr)
+      : "memory");
+}
+__device__ __forceinline__ void tmem_wait_load() { asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory"); }
+__device__ __forceinline__ void tmem_wait_store() { asm volatile("tcgen05.wait::st.sync.aligned;\n" ::: "memory"); }
 
 // Eight consecutive centroid values (fp16) of a lane's share of a packed row:
 // codes 8 J .. 8 J + 7 of the 32 the words hold.
-template <int BW, int J>
-__device__ __forceinline__ void decode_piece(const uint32_t (&w)[BW], uint32_t sel, uint32_t (&f)[4]) {
+template <int BW, int J, int NW>
+__device__ __forceinline__ void decode_piece(const uint32_t (&w)[NW], uint32_t sel, uint32_t (&f)[4]) {
   if constexpr (BW == 4) {
     f[0] = lut_byte<0>(w[J], sel); f[1] = lut_byte<1>(w[J], sel);
     f[2] = lut_byte<2>(w[J], sel); f[3] = lut_byte<3>(w[J], sel);
@@ -134,70 +211,117 @@ __device__ __forceinline__ void decode_piece(const uint32_t (&w)[BW], uint32_t s
     f[3] = join(lut_code<BW, 8 * J + 6>(w, sel), lut_code<BW, 8 * J + 7>(w, sel));
   }
 }
-
-// One warp decodes tokens 16 u .. 16 u + 15 of one side: the lane (g, t) takes
-// rows g and g + 8 and coordinates 32 t .. 32 t + 31 of each.
-// The values stored are centroid x row norm, rounded to fp16 (`norms` = address of the
-// tile's fp16 norms; rows from `valid` on get norm 0): the scores and the value sums then
-// need no per-token scaling.
-template <int BW>
-__device__ __forceinline__ void decode_group(uint32_t raw, uint32_t norms, int valid, uint32_t tile,
-                                             uint32_t sel, int u, int g, int t) {
-  constexpr int NB = 16 * BW;
+// The lane's quarter of a packed row in global memory.
+template <int BW, int NW> __device__ __forceinline__ void load_quarter(const uint8_t *at, uint32_t (&w)[NW]) {
+  if constexpr (BW == 6) {
 #pragma unroll
-  for (int h = 0; h < 2; ++h) {
-    const int row = 16 * u + g + 8 * h;
-    uint32_t w[BW];
-    load_words<4 * BW>(raw + (uint32_t)row * NB + (uint32_t)t * (4 * BW), w);
-    unsigned short nh;
-    asm volatile("ld.shared.u16 %0, [%1];\n" : "=h"(nh) : "r"(norms + 2u * row));
-    if (row >= valid) nh = 0;
-    const __half2 n2 = __half2half2(__ushort_as_half(nh));
-    auto scaled = [&](uint32_t x) {
-      const __half2 y = __hmul2(*reinterpret_cast<const __half2 *>(&x), n2);
-      return *reinterpret_cast<const uint32_t *>(&y);
-    };
-    uint32_t f[4];
-    decode_piece<BW, 0>(w, sel, f);
-    sts128(tile_at(tile, row, 4 * t + 0), scaled(f[0]), scaled(f[1]), scaled(f[2]), scaled(f[3]));
-    decode_piece<BW, 1>(w, sel, f);
-    sts128(tile_at(tile, row, 4 * t + 1), scaled(f[0]), scaled(f[1]), scaled(f[2]), scaled(f[3]));
-    decode_piece<BW, 2>(w, sel, f);
-    sts128(tile_at(tile, row, 4 * t + 2), scaled(f[0]), scaled(f[1]), scaled(f[2]), scaled(f[3]));
-    decode_piece<BW, 3>(w, sel, f);
-    sts128(tile_at(tile, row, 4 * t + 3), scaled(f[0]), scaled(f[1]), scaled(f[2]), scaled(f[3]));
+    for (int i = 0; i < 3; ++i) {
+      const uint2 v = __ldg(reinterpret_cast<const uint2 *>(at) + i);
+      w[2 * i] = v.x; w[2 * i + 1] = v.y;
+    }
+  } else {
+#pragma unroll
+    for (int i = 0; i < BW / 4; ++i) {
+      const uint4 v = __ldg(reinterpret_cast<const uint4 *>(at) + i);
+      w[4 * i] = v.x; w[4 * i + 1] = v.y; w[4 * i + 2] = v.z; w[4 * i + 3] = v.w;
+    }
   }
 }
 
-// fp32 dot products of one token's key centroids (row `at` of the landing
-// buffer) with four rotated query rows (null: the row does not exist), without
-// the key norm.  Out of line and returning its result in registers: it runs only
-// for tiles whose fp16 scores came out large and must cost the common path
-// neither registers nor stack.
-template <int BW>
-__device__ __noinline__ float4 precise_token(uint32_t at, const float *q0, const float *q1,
-                                             const float *q2, const float *q3,
-                                             const float *centroids) {
-  float4 r = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll 4
-  for (int d = 0; d < 128; ++d) {
-    const int bit = d * BW, b0 = bit >> 3, sh = bit & 7;
-    uint32_t x = lds_u8(at + b0);
-    if (sh + BW > 8) x |= lds_u8(at + b0 + 1) << 8;
-    const float cv = __ldg(centroids + ((x >> sh) & ((1u << BW) - 1u)));
-    r.x = fmaf(q0 ? __ldg(q0 + d) : 0.f, cv, r.x);
-    r.y = fmaf(q1 ? __ldg(q1 + d) : 0.f, cv, r.y);
-    r.z = fmaf(q2 ? __ldg(q2 + d) : 0.f, cv, r.z);
-    r.w = fmaf(q3 ? __ldg(q3 + d) : 0.f, cv, r.w);
+__device__ __forceinline__ uint32_t times(uint32_t c, __half2 n) {
+  const __half2 y = __hmul2(*reinterpret_cast<const __half2 *>(&c), n);
+  return *reinterpret_cast<const uint32_t *>(&y);
+}
+// Tokens 16 u .. 16 u + 15 of a tile: the lane (g, t) stores rows g and g + 8, coordinates
+// 32 t .. 32 t + 31, as centroid x row norm rounded to fp16 (the scores and value sums then
+// need no per-token scaling).
+template <int BW, int NW>
+__device__ __forceinline__ void decode_task(uint32_t tile, int u, int g, int t, uint32_t sel,
+                                            const uint32_t (&w)[2][NW], const __half (&nrm)[2]) {
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const int row = 16 * u + g + 8 * h;
+    const __half2 n = __half2half2(nrm[h]);
+    uint32_t f[4];
+    decode_piece<BW, 0>(w[h], sel, f);
+    sts128(operand_at(tile, row, 4 * t + 0), times(f[0], n), times(f[1], n), times(f[2], n), times(f[3], n));
+    decode_piece<BW, 1>(w[h], sel, f);
+    sts128(operand_at(tile, row, 4 * t + 1), times(f[0], n), times(f[1], n), times(f[2], n), times(f[3], n));
+    decode_piece<BW, 2>(w[h], sel, f);
+    sts128(operand_at(tile, row, 4 * t + 2), times(f[0], n), times(f[1], n), times(f[2], n), times(f[3], n));
+    decode_piece<BW, 3>(w[h], sel, f);
+    sts128(operand_at(tile, row, 4 * t + 3), times(f[0], n), times(f[1], n), times(f[2], n), times(f[3], n));
   }
-  return r;
+}
+
+// fp32 scores of this thread's query row against the 64 tokens of a tile, written over the
+// tile's scores in tensor memory (`s_addr`, lane base included): the packed codes of its kv head are read
+// from the pages (the same address for the whole warp) and the row of `q` along with them.
+// Out of line: it runs only for tiles whose fp16 scores came out large.
+template <int BW>
+__device__ __noinline__ void precise_tile(const uint8_t *pages, int64_t page_stride, const __half *all_norms,
+                                          int64_t norm_page_stride, const float *centroids, const int32_t *table,
+                                          int P, int S, int tok0, int end, const float *q, uint32_t s_addr) {
+  const int shift = 31 - __clz(S);
+#pragma unroll 1
+  for (int blk = 0; blk < kTile / 16; ++blk) {                // sixteen tokens of one page
+    const int tok = tok0 + 16 * blk;
+    const int page = tok < end ? table[tok >> shift] : -1;
+    float acc[16];
+#pragma unroll
+    for (int i = 0; i < 16; ++i) acc[i] = 0.f;
+    if (page >= 0 && page < P) {
+      const int pos = tok & (S - 1);
+      const uint8_t *row = pages + (int64_t)page * page_stride + (int64_t)pos * (16 * BW);
+#pragma unroll 1
+      for (int d = 0; d < 32; ++d) {                           // four coordinates: BW / 2 bytes of each row
+        const float4 x = q ? __ldg(reinterpret_cast<const float4 *>(q) + d) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+          uint32_t w = 0;
+#pragma unroll
+          for (int b = 0; b < BW / 2; ++b) w |= (uint32_t)__ldg(row + i * (16 * BW) + d * (BW / 2) + b) << (8 * b);
+          constexpr uint32_t kMask = (1u << BW) - 1u;
+          acc[i] = fmaf(x.x, __ldg(centroids + (w & kMask)), acc[i]);
+          acc[i] = fmaf(x.y, __ldg(centroids + ((w >> BW) & kMask)), acc[i]);
+          acc[i] = fmaf(x.z, __ldg(centroids + ((w >> (2 * BW)) & kMask)), acc[i]);
+          acc[i] = fmaf(x.w, __ldg(centroids + ((w >> (3 * BW)) & kMask)), acc[i]);
+        }
+      }
+      const __half *norms = all_norms + (int64_t)page * norm_page_stride + pos;
+#pragma unroll
+      for (int i = 0; i < 16; ++i) acc[i] *= __half2float(norms[i]);
+    }
+    uint32_t v[16];
+#pragma unroll
+    for (int i = 0; i < 16; ++i) v[i] = __float_as_uint(acc[i]);
+    __syncwarp();
+    tmem_store16(s_addr + 16 * blk, v);
+  }
+  tmem_wait_store();
+}
+
+// Scores of the tokens from `seen` on become -inf (`masked`: some row of the warp has
+// such); returns the row's maximum.
+__device__ __forceinline__ float mask_and_maximum(uint32_t (&s)[64], bool masked, int seen) {
+  if (masked) {
+#pragma unroll
+    for (int i = 0; i < 64; ++i) s[i] = i >= seen ? 0xff800000u : s[i];
+  }
+  float a = -INFINITY, c = -INFINITY;
+#pragma unroll
+  for (int i = 0; i < 64; i += 4) {
+    a = max3(a, __uint_as_float(s[i]), __uint_as_float(s[i + 1]));
+    c = max3(c, __uint_as_float(s[i + 2]), __uint_as_float(s[i + 3]));
+  }
+  return fmaxf(a, c);
 }
 
 template <int BWK, int BWV>
 __global__ void __launch_bounds__(kThreads, 1) prefill_kernel(Params p) {
   using M = Map<BWK, BWV>;
   extern __shared__ __align__(128) uint8_t dyn_smem[];
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   if ((uint32_t)__cvta_generic_to_shared(dyn_smem) > kBase) {   // layout assumption broken
     if (p.status && tid == 0) atomicOr(p.status, WTQ_STATUS_LAYOUT);
     return;
@@ -210,22 +334,36 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_kernel(Params p) {
     const int len = L - p.Q + 1 + i % p.Q;
     p.row_lens[i] = len < 0 ? 0 : len;
   }
-  // lookup tables (built by the rotation launch)
+  // lookup tables (built by the rotation launch), tensor memory, barriers
   for (int i = tid; i < (int)(M::kLutBytes / 16); i += kThreads) {
     const uint4 v = __ldg(reinterpret_cast<const uint4 *>(p.lut) + i);
     sts128(mma::kLutAddr + 16u * i, v.x, v.y, v.z, v.w);
   }
-  const uint32_t sel_k = mma::kLutAddr | (uint32_t)(lane << 2), sel_v = sel_k | 0x80u;
-  // ldmatrix row addresses of this lane.  A piece index is 2 * step + (0 or 1) and
-  // the swizzle XORs it with the row's low bits, so the step enters as one XOR of
-  // step << 5 with these bases; steps over rows of 16 leave the low bits alone.
-  const uint32_t q_at = tile_at(M::kQTile, 32 * warp + (lane & 7) + 8 * ((lane >> 3) & 1), lane >> 4);
-  const uint32_t k_at = tile_at(kKTile, (lane & 7) + 8 * (lane >> 4), (lane >> 3) & 1);
-  const uint32_t v_at = tile_at(kVTile, (lane & 7) + 8 * ((lane >> 3) & 1), lane >> 4);
+  if (warp == kMmaWarp) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(kTmemSlot),
+                 "r"(kCols) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
+  }
+  if (tid == 0) {
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(kKFull + 8u * i, 4);                        // the four 16-token groups of a tile
+      mbar_init(kVFull + 8u * i, 4);
+      mbar_init(kKFree + 8u * i, 1);
+      mbar_init(kVFree + 8u * i, 1);
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      mbar_init(kSFull + 8u * i, 1);
+      mbar_init(kODone + 8u * i, 1);
+      mbar_init(kPFull + 8u * i, 4);                        // the four warps of an M tile
+    }
+    sts32(kAbort, 0u);
+    asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+  }
   const int R = p.Q * p.n_rep;                              // query rows per (sequence, kv head)
   const int items = p.B * p.Hkv * p.row_blocks * p.num_splits;
   const int page_shift = 31 - __clz(p.S);
-
   // ---- balanced schedule ---------------------------------------------------------------
   // The 64-token tiles of all groups, laid end to end (sequence, row block, kv head), are
   // cut into one equal run per block, so every multiprocessor gets the same number of
@@ -273,9 +411,18 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_kernel(Params p) {
   auto walk64 = [&](uint32_t at) -> long long {
     return (long long)(((unsigned long long)lds32(at + 4) << 32) | lds32(at));
   };
+  fence_before();
+  __syncthreads();
+  fence_after();
+  const uint32_t tmem = lds32(kTmemSlot);
+  // Tiles handled so far, over all items: buffers alternate and barrier phases count on.
+  int tiles_all = 0, tiles_m[2] = {0, 0};
 
   for (;;) {
+    fence_before();
     __syncthreads();                                        // everyone is done with the previous item
+    fence_after();
+    if (lds32(kAbort) != 0u) break;
     if (tid == 0) {
       if (!p.balanced) {
         sts32(kItem, (uint32_t)atomicAdd(p.work_counter, 1));
@@ -343,324 +490,267 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_kernel(Params p) {
       const int len = L - p.Q + 1 + row / p.n_rep;
       return len < 0 ? 0 : len;
     };
-    const int len_last = length_of(row_hi - 1);
-    if (row_lo >= R || start >= len_last) continue;         // no row of the block sees this chunk
-    const int end = min(cap, len_last);
-    const int ntiles = (end - start + kTile - 1) / kTile;
-
-    // ---- this lane's four rows ------------------------------------------------
-    const int wrow0 = row_lo + 32 * warp;
-    int limit[2][2];                                        // first token a row does NOT see, within the chunk
-#pragma unroll
-    for (int m = 0; m < 2; ++m)
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const int row = wrow0 + 16 * m + 8 * h + g;
-        limit[m][h] = min(row < row_hi ? length_of(row) : 0, cap);
-      }
-    // index of a row's rotated query (and, times num_splits, of its chunk states); -1: no such row
-    auto query_row = [&](int m, int h) -> int64_t {
-      const int row = wrow0 + 16 * m + 8 * h + g;
-      if (row >= row_hi) return -1;
-      const int i = row / p.n_rep, r = row - i * p.n_rep;
-      return ((int64_t)b * p.Q + i) * p.Hq + kvh * p.n_rep + r;
-    };
-    // rows are in causal order: the warp's first and last existing rows bound its limits
-    const int warp_hi = wrow0 < row_hi ? min(length_of(min(wrow0 + 31, row_hi - 1)), cap) : 0;
-    const int warp_lo = wrow0 < row_hi ? min(length_of(wrow0), cap) : 0;
-    const bool warp_on = warp_hi > start;
-
-    // ---- copy of one tile into a landing buffer ----------------------------------
-    // Done in two steps so that the page-table reads are not in front of the
-    // copies: `lookup(j)` fetches the page id of each of this thread's pieces of
-    // tile j into registers (at the top of tile j - 1's turn), `copy(j)` issues
-    // the copies after that tile has been decoded.
-    const int32_t *table = p.page_table + (int64_t)b * p.table_stride;
-    constexpr int kPiecesK = kTile * M::kNBK / 16, kPiecesV = kTile * M::kNBV / 16;
-    constexpr int kPieces = kPiecesK + kPiecesV + 16;       // + 8 + 8 pieces of norms
-    constexpr int kTurns = (kPieces + kThreads - 1) / kThreads;
-    // piece c: side 0/1 = K/V codes, 2/3 = K/V norms; first token; byte offset in the row
-    auto piece = [&](int c, int &side, int &tok, int &off, uint32_t &dst) {
-      if (c < kPiecesK) {
-        side = 0; tok = c / (M::kNBK / 16); off = (c - tok * (M::kNBK / 16)) * 16; dst = 16u * c;
-      } else if (c < kPiecesK + kPiecesV) {
-        const int cc = c - kPiecesK;
-        side = 1; tok = cc / (M::kNBV / 16); off = (cc - tok * (M::kNBV / 16)) * 16;
-        dst = M::kRawV + 16u * cc;
-      } else {
-        const int cc = c - kPiecesK - kPiecesV;              // eight tokens of norms per piece
-        side = 2 + (cc >> 3); tok = (cc & 7) * 8; off = 0;
-        dst = (side == 2 ? M::kRawNK : M::kRawNV) + 16u * (cc & 7);
-      }
-    };
-    int page_of[kTurns];                                     // -2: the piece lies past the end
-    auto lookup = [&](int j) {
-#pragma unroll
-      for (int i = 0; i < kTurns; ++i) {
-        const int c = tid + i * kThreads;
-        int side, tok, off;
-        uint32_t dst;
-        piece(c < kPieces ? c : 0, side, tok, off, dst);
-        const int token = start + j * kTile + tok;
-        page_of[i] = c < kPieces && token < end ? table[token >> page_shift] : -2;
-      }
-    };
-    auto copy = [&](int j) {
-      const uint32_t raw = M::kRaw + (uint32_t)(j & 1) * M::kRawBytes;
-#pragma unroll
-      for (int i = 0; i < kTurns; ++i) {
-        const int c = tid + i * kThreads;
-        if (c >= kPieces) break;
-        int side, tok, off;
-        uint32_t dst;
-        piece(c, side, tok, off, dst);
-        const int page = page_of[i], pos = (start + j * kTile + tok) & (p.S - 1);
-        int bytes = 16;
-        const void *src = p.k.pages;                         // any valid address when nothing is read
-        if (page < 0 || page >= p.P) {
-          if (page != -2 && p.status) atomicOr(p.status, WTQ_STATUS_BAD_PAGE);
-          bytes = 0;
-        } else if (side < 2) {
-          const DecodeSideDev &sd = side ? p.v : p.k;
-          src = sd.pages + (int64_t)page * sd.page_stride + (int64_t)kvh * sd.head_stride +
-                (int64_t)pos * sd.nb + off;
-        } else {
-          const DecodeSideDev &sd = side == 3 ? p.v : p.k;
-          src = sd.norms + (int64_t)page * sd.norm_page_stride + (int64_t)kvh * sd.norm_head_stride + pos;
-        }
-        copy16(raw + dst, src, bytes);
-      }
-      asm volatile("cp.async.commit_group;\n" ::: "memory");
-    };
-    lookup(0);
-    copy(0);
-    if (ntiles > 1) lookup(1);
-
-    // ---- query rows -> fp16 tile (behind the first copy, eight loads in flight per thread) ----
-    for (int e0 = tid; e0 < kRows * 32; e0 += 8 * kThreads) {  // 32 float4 per row
-      float4 v[8];
-#pragma unroll
-      for (int u = 0; u < 8; ++u) {
-        const int e = e0 + u * kThreads, lr = e >> 5, c4 = e & 31, row = row_lo + lr;
-        v[u] = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (row < row_hi) {
-          const int i = row / p.n_rep, r = row - i * p.n_rep;
-          const int64_t qrow = ((int64_t)b * p.Q + i) * p.Hq + kvh * p.n_rep + r;
-          v[u] = __ldg(reinterpret_cast<const float4 *>(p.q_rot + qrow * 128) + c4);
-        }
-      }
-#pragma unroll
-      for (int u = 0; u < 8; ++u) {
-        const int e = e0 + u * kThreads, lr = e >> 5, c4 = e & 31;
-        sts64u(tile_at(M::kQTile, lr, c4 >> 1) + (uint32_t)(c4 & 1) * 8u, pack_half2(v[u].x, v[u].y),
-               pack_half2(v[u].z, v[u].w));
-      }
-    }
-
-    float o[2][16][4];                                      // rows x coordinates of the value basis
-    float mx[2][2], sum[2][2];
+    if (row_lo >= R) continue;
+    // tiles each of the two M tiles sees (rows are in causal order: its last row sees most)
+    int ntiles[2];
 #pragma unroll
     for (int m = 0; m < 2; ++m) {
-#pragma unroll
-      for (int n = 0; n < 16; ++n)
-#pragma unroll
-        for (int e = 0; e < 4; ++e) o[m][n][e] = 0.f;
-      mx[m][0] = mx[m][1] = -INFINITY;
-      sum[m][0] = sum[m][1] = 0.f;
+      const int last = min(row_hi, row_lo + 128 * (m + 1)) - 1;
+      const int limit = last >= row_lo + 128 * m ? min(length_of(last), cap) : 0;
+      ntiles[m] = limit > start ? (limit - start + kTile - 1) / kTile : 0;
     }
+    const int end = min(cap, length_of(row_hi - 1));
+    const int nt = max(ntiles[0], ntiles[1]);
+    if (nt == 0) continue;                                  // no row of the block sees this range
+    const int32_t *table = p.page_table + (int64_t)b * p.table_stride;
 
-    for (int j = 0; j < ntiles; ++j) {
-      const uint32_t raw = M::kRaw + (uint32_t)(j & 1) * M::kRawBytes;
-      const int tok0 = start + j * kTile;
-      asm volatile("cp.async.wait_group 0;\n" ::: "memory");
-      __syncthreads();       // the tile has landed for everyone; everyone is done with the previous tiles
-      // ---- decode: warps 0..3 the four key groups, warps 4..7 the value groups ------
-      // (norms are copied eight tokens at a time: those of tokens past the end of
-      // the tile's range are whatever the page holds and become 0 here)
-      if (warp < 4) {
-        decode_group<BWK>(raw, raw + M::kRawNK, end - tok0, kKTile, sel_k, warp, g, t);
-        if (lane < 16) {                                     // fp32 norms, for the fp32 re-scoring only
-          const int tk = 16 * warp + lane;
-          const float v = tok0 + tk < end ? lds_half(raw + M::kRawNK + 2u * tk) : 0.f;
-          sts32(kNormK + 4u * tk, __float_as_uint(v));
+    // ---- query rows -> fp16 operand (the softmax warps; the decode warps start at once) ----
+    if (warp < kSoftWarps) {
+      const int most = ntiles[1] > 0 ? 4096 : 2048;          // (row, piece) units
+#pragma unroll 4
+      for (int u = tid; u < most; u += 32 * kSoftWarps) {
+        const int piece = (u >> 3) & 15, lr = (u & 7) + 8 * (u >> 7), row = row_lo + lr;
+        float4 x = make_float4(0.f, 0.f, 0.f, 0.f), y = x;
+        if (row < row_hi) {
+          const int i = row / p.n_rep, r = row - i * p.n_rep;
+          const float4 *src = reinterpret_cast<const float4 *>(
+              p.q_rot + (((int64_t)b * p.Q + i) * p.Hq + kvh * p.n_rep + r) * 128 + 8 * piece);
+          x = __ldg(src);
+          y = __ldg(src + 1);
         }
-      } else {
-        decode_group<BWV>(raw + M::kRawV, raw + M::kRawNV, end - tok0, kVTile, sel_v, warp - 4, g, t);
+        sts128(operand_at(M::kQTile, lr, piece), pack_half2(x.x, x.y), pack_half2(x.z, x.w), pack_half2(y.x, y.y),
+               pack_half2(y.z, y.w));
       }
-      __syncthreads();
-      if (j + 1 < ntiles) copy(j + 1);
-      if (j + 2 < ntiles) lookup(j + 2);                    // ids for the tile after: a whole tile ahead
-      if (!warp_on || tok0 >= warp_hi) continue;            // no row of this warp sees the tile
+      asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+    }
+    if (warp < kSoftWarps || warp == kMmaWarp)
+      asm volatile("bar.sync 1, %0;\n" ::"r"(32 * (kSoftWarps + 1)) : "memory");
 
-      // ---- scores -------------------------------------------------------------------
-      float s[2][8][4];
+    if (warp < kSoftWarps) {
+      // ================= softmax: M tile m, one query row per thread ====================
+      const int m = warp >> 2;
+      const uint32_t lanes = (uint32_t)(32 * (warp & 3)) << 16;
+      const int row = row_lo + 128 * m + 32 * (warp & 3) + lane;
+      const int limit = row < row_hi ? min(length_of(row), cap) : 0;   // first token the row does NOT see
+      int64_t qrow = -1;
+      if (row < row_hi) {
+        const int i = row / p.n_rep, r = row - i * p.n_rep;
+        qrow = ((int64_t)b * p.Q + i) * p.Hq + kvh * p.n_rep + r;
+      }
+      const int all_see = __reduce_min_sync(kFull, limit);             // every row of the warp sees the tokens below
+      const int n = ntiles[m];
+      float ref = -INFINITY, sum = 0.f;
+      bool ok = true;
+      for (int j = 0; j < n && ok; ++j) {
+        const int T = tiles_m[m] + j, buf = T & 1, tok0 = start + j * kTile;
+        const uint32_t s_addr = tmem + lanes + kColS + 128u * m + 64u * buf;
+        ok = mbar_wait(kSFull + 16u * m + 8u * buf, T >> 1);
+        if (!__all_sync(kFull, ok)) { ok = false; break; }
+        fence_after();
+        uint32_t s[64];
+        tmem_load32<0>(s_addr, s);
+        tmem_load32<32>(s_addr + 32, s);
+        tmem_wait_load();
+        float mx = mask_and_maximum(s, tok0 + kTile > all_see, limit - tok0);
+        // The fp16 error of a score grows with its size, and only scores near their row's
+        // maximum carry weight: a tile is re-scored in fp32 when a row maximum lies beyond
+        // +-8 (or is not a number).
+        if (__any_sync(kFull, !(fabsf(mx) <= kPreciseAbove) && mx != -INFINITY)) {
+          precise_tile<BWK>(p.k.pages + (int64_t)kvh * p.k.head_stride, p.k.page_stride,
+                            p.k.norms + (int64_t)kvh * p.k.norm_head_stride, p.k.norm_page_stride, p.k.centroids, table,
+                            p.P, p.S, tok0, end, qrow < 0 ? nullptr : p.q_rot + qrow * 128, s_addr);
+          tmem_load32<0>(s_addr, s);
+          tmem_load32<32>(s_addr + 32, s);
+          tmem_wait_load();
+          mx = mask_and_maximum(s, tok0 + kTile > all_see, limit - tok0);
+        }
+        if (__any_sync(kFull, mx > ref + kSlack || (ref == -INFINITY && mx != -INFINITY))) {
+          const float now = mx > ref + kSlack || ref == -INFINITY ? mx : ref;
+          if (j > 0) {                                                  // rescale what is accumulated
+            const float scale = ref == now ? 1.f : ref == -INFINITY ? 0.f : ex2(ref - now);
+            sum *= scale;
+            ok = mbar_wait(kODone + 16u * m + 8u * (buf ^ 1), (T - 1) >> 1);
+            if (!__all_sync(kFull, ok)) { ok = false; break; }
+            fence_after();
+#pragma unroll 1
+            for (int c0 = 0; c0 < 128; c0 += 32) {
+              uint32_t o[32];
+              const uint32_t o_addr = tmem + lanes + kColO + 128u * m + c0;
+              tmem_load32<0>(o_addr, o);
+              tmem_wait_load();
 #pragma unroll
-      for (int m = 0; m < 2; ++m)
+              for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * scale);
+              tmem_store32(o_addr, o);
+            }
+            tmem_wait_store();
+          }
+          ref = now;
+        }
+        const float base = ref == -INFINITY ? 0.f : ref;
+        uint32_t pr[32];
+        float sa = 0.f, sb = 0.f;
 #pragma unroll
-        for (int n = 0; n < 8; ++n)
+        for (int i = 0; i < 32; ++i) {
+          const float x = ex2(__uint_as_float(s[2 * i]) - base), y = ex2(__uint_as_float(s[2 * i + 1]) - base);
+          sa += x;
+          sb += y;
+          pr[i] = pack_half2(x, y);
+        }
+        sum += sa + sb;
+        tmem_store32(s_addr, pr);                                       // over the scores just read
+        tmem_wait_store();
+        fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(kPFull + 16u * m + 8u * buf);
+      }
+      // ---- the rows' states -----------------------------------------------------------
+      if (ok && n > 0) {
+        const int last = tiles_m[m] + n - 1;
+        ok = mbar_wait(kODone + 16u * m + 8u * (last & 1), last >> 1);
+        if (__all_sync(kFull, ok)) {
+          fence_after();
+          const bool keep = qrow >= 0 && limit > start;                 // the row exists and sees part of the range
+          const int64_t state = qrow * p.num_splits + chunk;
+#pragma unroll 1
+          for (int c0 = 0; c0 < 128; c0 += 32) {
+            uint32_t o[32];
+            tmem_load32<0>(tmem + lanes + kColO + 128u * m + c0, o);
+            tmem_wait_load();
+            if (keep) {
+              uint4 *dst = reinterpret_cast<uint4 *>(p.part_acc + state * 128 + c0);
 #pragma unroll
-          for (int e = 0; e < 4; ++e) s[m][n][e] = 0.f;
-#pragma unroll
-      for (int ks = 0; ks < 8; ++ks) {
-        uint32_t a[2][4];
-#pragma unroll
-        for (int m = 0; m < 2; ++m) ldmatrix_x4((q_at + m * 16 * 256) ^ (uint32_t)(ks << 5), a[m]);
-#pragma unroll
-        for (int np = 0; np < 4; ++np) {
-          uint32_t kb[4];
-          ldmatrix_x4((k_at + np * 16 * 256) ^ (uint32_t)(ks << 5), kb);
-#pragma unroll
-          for (int m = 0; m < 2; ++m) {
-            mma16816_free(s[m][2 * np], a[m][0], a[m][1], a[m][2], a[m][3], kb[0], kb[1]);
-            mma16816_free(s[m][2 * np + 1], a[m][0], a[m][1], a[m][2], a[m][3], kb[2], kb[3]);
+              for (int i = 0; i < 8; ++i) dst[i] = make_uint4(o[4 * i], o[4 * i + 1], o[4 * i + 2], o[4 * i + 3]);
+            }
+          }
+          if (keep) {
+            p.part_m[state] = ref;
+            p.part_l[state] = sum;
           }
         }
       }
-      const bool masked = tok0 + kTile > warp_lo;            // some row of the warp stops inside the tile
-      if (masked) {
-#pragma unroll
-        for (int m = 0; m < 2; ++m)
-#pragma unroll
-          for (int n = 0; n < 8; ++n)
-#pragma unroll
-            for (int e = 0; e < 4; ++e)
-              if (tok0 + 8 * n + 2 * t + (e & 1) >= limit[m][e >> 1]) s[m][n][e] = -INFINITY;
-      }
-      float ref[2][2];                                       // maxima of the tile's rows
-      auto row_maxima = [&]() {
-#pragma unroll
-        for (int m = 0; m < 2; ++m)
+    } else if (warp < kMmaWarp) {
+      // ================= decode ==========================================================
+      // Tasks of 16 tokens of one side, eight per tile (four of K, four of V), dealt round-robin;
+      // the codes of a warp's next task are on their way while it decodes this one.
+      constexpr int kMost = BWK > BWV ? BWK : BWV;
+      const int g = lane & 7, t = lane >> 3;
+      const uint32_t sel = mma::kLutAddr | (uint32_t)(lane << 2);
+      const int tasks = 8 * nt;
+      auto page_of = [&](int q) {                                       // -2: past the end of the range
+        const int tok = start + (q >> 3) * kTile + 16 * (q & 3);
+        return q < tasks && tok < end ? table[tok >> page_shift] : -2;
+      };
+      auto load = [&](int q, int page, uint32_t (&w)[2][kMost], __half (&nrm)[2]) {
+        const bool is_v = (q & 4) != 0;
+        const DecodeSideDev &sd = is_v ? p.v : p.k;
+        const int tok = start + (q >> 3) * kTile + 16 * (q & 3);
+        if ((uint32_t)page < (uint32_t)p.P) {
+          const int pos = tok & (p.S - 1);
+          const uint8_t *rows = sd.pages + (int64_t)page * sd.page_stride + (int64_t)kvh * sd.head_stride;
+          const __half *norms = sd.norms + (int64_t)page * sd.norm_page_stride + (int64_t)kvh * sd.norm_head_stride + pos;
 #pragma unroll
           for (int h = 0; h < 2; ++h) {
-            float v = -INFINITY;
-#pragma unroll
-            for (int n = 0; n < 8; ++n) v = max3(v, s[m][n][2 * h], s[m][n][2 * h + 1]);
-            v = fmaxf(v, __shfl_xor_sync(kFull, v, 1));
-            ref[m][h] = fmaxf(v, __shfl_xor_sync(kFull, v, 2));
+            const int r = g + 8 * h;
+            if (BWK == BWV || !is_v) {
+              load_quarter<BWK>(rows + (int64_t)(pos + r) * (16 * BWK) + t * (4 * BWK), w[h]);
+            } else {
+              load_quarter<BWV>(rows + (int64_t)(pos + r) * (16 * BWV) + t * (4 * BWV), w[h]);
+            }
+            nrm[h] = norms[r];
+            if (tok + r >= end) nrm[h] = __ushort_as_half(0);
           }
-      };
-      row_maxima();
-      // The fp16 error of a score grows with its size, and only scores near their
-      // row's maximum carry weight: a tile is re-scored in fp32 when a row maximum
-      // lies beyond +-8 (or is not a number).
-      bool large = false;
-#pragma unroll
-      for (int m = 0; m < 2; ++m)
-#pragma unroll
-        for (int h = 0; h < 2; ++h) large |= !(fabsf(ref[m][h]) <= kPreciseAbove) && ref[m][h] != -INFINITY;
-      if (__any_sync(kFull, large)) {
-        const float *qp[4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const int64_t qr = query_row(i >> 1, i & 1);
-          qp[i] = qr < 0 ? nullptr : p.q_rot + qr * 128;
-        }
-#pragma unroll
-        for (int n = 0; n < 8; ++n)
-#pragma unroll
-          for (int c = 0; c < 2; ++c) {
-            const int tk = 8 * n + 2 * t + c;
-            const float4 r = precise_token<BWK>(raw + (uint32_t)tk * M::kNBK, qp[0], qp[1], qp[2], qp[3],
-                                                p.k.centroids);
-            const float nk_tk = __uint_as_float(lds32(kNormK + 4u * tk));
-            const float x[4] = {r.x, r.y, r.z, r.w};
-#pragma unroll
-            for (int m = 0; m < 2; ++m)
-#pragma unroll
-              for (int h = 0; h < 2; ++h)
-                s[m][n][2 * h + c] = masked && tok0 + tk >= limit[m][h] ? -INFINITY
-                                                                        : x[2 * m + h] * nk_tk;
-          }
-        row_maxima();
-      }
-
-      // ---- online softmax -------------------------------------------------------------
-      bool grew = false;
-#pragma unroll
-      for (int m = 0; m < 2; ++m)
-#pragma unroll
-        for (int h = 0; h < 2; ++h) grew |= ref[m][h] > mx[m][h];
-      if (__any_sync(kFull, grew)) {
-#pragma unroll
-        for (int m = 0; m < 2; ++m) {
-          float scale[2];
+        } else {
+          if (page != -2 && p.status && lane == 0) atomicOr(p.status, WTQ_STATUS_BAD_PAGE);
 #pragma unroll
           for (int h = 0; h < 2; ++h) {
-            const float now = fmaxf(mx[m][h], ref[m][h]);
-            scale[h] = now == -INFINITY ? 1.f : ex2(mx[m][h] - now);   // ex2(-inf) = 0 on the first tile
-            mx[m][h] = now;
-            sum[m][h] *= scale[h];
+#pragma unroll
+            for (int k = 0; k < kMost; ++k) w[h][k] = 0u;
+            nrm[h] = __ushort_as_half(0);
           }
-#pragma unroll
-          for (int n = 0; n < 16; ++n) {
-            o[m][n][0] *= scale[0]; o[m][n][1] *= scale[0];
-            o[m][n][2] *= scale[1]; o[m][n][3] *= scale[1];
-          }
-        }
-      }
-      uint32_t pa[2][8][2];                                  // P * value norm as fp16 pairs
-      float base[2][2];
-#pragma unroll
-      for (int m = 0; m < 2; ++m)
-#pragma unroll
-        for (int h = 0; h < 2; ++h) base[m][h] = mx[m][h] == -INFINITY ? 0.f : mx[m][h];
-      auto probabilities = [&](int n) {                      // of tokens 8 n .. 8 n + 7
-#pragma unroll
-        for (int m = 0; m < 2; ++m) {
-          const float p0 = ex2(s[m][n][0] - base[m][0]), p1 = ex2(s[m][n][1] - base[m][0]);
-          const float p2 = ex2(s[m][n][2] - base[m][1]), p3 = ex2(s[m][n][3] - base[m][1]);
-          sum[m][0] += p0 + p1;
-          sum[m][1] += p2 + p3;
-          pa[m][n][0] = pack_half2(p0, p1);
-          pa[m][n][1] = pack_half2(p2, p3);
         }
       };
-
-      // ---- values: in source order the probabilities of the next 16 tokens sit
-      // between the MMAs of the current 16 (the compiler is free to schedule the
-      // exponentials under the tensor pipe's work; measured, it made no difference)
-      probabilities(0);
-      probabilities(1);
+      uint32_t w[2][kMost], next[2][kMost];
+      __half nrm[2], nrm_next[2];
+      int q = warp - kSoftWarps;
+      if (q < tasks) load(q, page_of(q), w, nrm);
+      int page = page_of(q + kDecodeWarps);
+      for (; q < tasks; q += kDecodeWarps) {
+        if (q + kDecodeWarps < tasks) load(q + kDecodeWarps, page, next, nrm_next);
+        page = page_of(q + 2 * kDecodeWarps);
+        const bool is_v = (q & 4) != 0;
+        const int T = tiles_all + (q >> 3), buf = T & 1, u = q & 3;
+        if (T >= 2) {                                                   // the tile's last reader is done
+          const bool ok = mbar_wait((is_v ? kVFree : kKFree) + 8u * buf, (T >> 1) - 1);
+          if (!__all_sync(kFull, ok)) break;
+        }
+        if (!is_v) decode_task<BWK>(M::kKTile + (uint32_t)buf * kTileBytes, u, g, t, sel, w, nrm);
+        else decode_task<BWV>(kVTile + (uint32_t)buf * kTileBytes, u, g, t, sel | 0x80u, w, nrm);
+        asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+        __syncwarp();
+        if (lane == 0) mbar_arrive((is_v ? kVFull : kKFull) + 8u * buf);
 #pragma unroll
-      for (int kk = 0; kk < 4; ++kk) {
+        for (int h = 0; h < 2; ++h) {
 #pragma unroll
-        for (int dp = 0; dp < 8; ++dp) {
-          uint32_t vb[4];
-          ldmatrix_x4_trans((v_at + kk * 16 * 256) ^ (uint32_t)(dp << 5), vb);
+          for (int k = 0; k < kMost; ++k) w[h][k] = next[h][k];
+          nrm[h] = nrm_next[h];
+        }
+      }
+    } else if (lane == 0) {
+      // ================= multiply: one thread ============================================
+      bool ok = true;
+      for (int j = 0; j <= nt && ok; ++j) {
+        if (j < nt) {                                                   // scores of tile j
+          const int T = tiles_all + j, buf = T & 1;
+          ok = mbar_wait(kKFull + 8u * buf, T >> 1);
+          for (int m = 0; m < 2 && ok; ++m) {
+            if (j >= ntiles[m]) continue;
+            const int Tm = tiles_m[m] + j, sb = Tm & 1;
+            // the buffer's last probabilities have been consumed (those of an earlier item were
+            // before its states were written)
+            if (j >= 2) ok = mbar_wait(kODone + 16u * m + 8u * sb, (Tm - 2) >> 1);
+            if (!ok) break;
+            fence_after();
+            const uint32_t d = tmem + kColS + 128u * m + 64u * sb;
 #pragma unroll
-          for (int m = 0; m < 2; ++m) {
-            mma16816_free(o[m][2 * dp], pa[m][2 * kk][0], pa[m][2 * kk][1], pa[m][2 * kk + 1][0],
-                     pa[m][2 * kk + 1][1], vb[0], vb[1]);
-            mma16816_free(o[m][2 * dp + 1], pa[m][2 * kk][0], pa[m][2 * kk][1], pa[m][2 * kk + 1][0],
-                     pa[m][2 * kk + 1][1], vb[2], vb[3]);
+            for (int ks = 0; ks < 8; ++ks)
+              umma_ss(d, desc_k_major(M::kQTile + (uint32_t)m * 32768u, ks),
+                      desc_k_major(M::kKTile + (uint32_t)buf * kTileBytes, ks), kIdescQK, ks > 0);
+            umma_commit(kSFull + 16u * m + 8u * sb);
           }
-          if (kk < 3 && dp == 1) probabilities(2 * kk + 2);
-          if (kk < 3 && dp == 5) probabilities(2 * kk + 3);
+          if (ok) umma_commit(kKFree + 8u * buf);
+        }
+        if (j > 0 && ok) {                                              // values of tile j - 1
+          const int i = j - 1, T = tiles_all + i, buf = T & 1;
+          ok = mbar_wait(kVFull + 8u * buf, T >> 1);
+          for (int m = 0; m < 2 && ok; ++m) {
+            if (i >= ntiles[m]) continue;
+            const int Tm = tiles_m[m] + i;
+            ok = mbar_wait(kPFull + 16u * m + 8u * (Tm & 1), Tm >> 1);
+            if (!ok) break;
+            fence_after();
+            const uint32_t a = tmem + kColS + 128u * m + 64u * (Tm & 1), d = tmem + kColO + 128u * m;
+#pragma unroll
+            for (int ks = 0; ks < 4; ++ks)
+              umma_ts(d, a + 8u * ks, desc_mn_major(kVTile + (uint32_t)buf * kTileBytes, ks), kIdescPV, i > 0 || ks > 0);
+            umma_commit(kODone + 16u * m + 8u * (Tm & 1));
+          }
+          if (ok) umma_commit(kVFree + 8u * buf);
         }
       }
     }
-
-    // ---- chunk states ---------------------------------------------------------------------
-#pragma unroll
-    for (int m = 0; m < 2; ++m)
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        float l = sum[m][h];
-        l += __shfl_xor_sync(kFull, l, 1);
-        l += __shfl_xor_sync(kFull, l, 2);
-        const int64_t qr = query_row(m, h);
-        if (qr < 0 || limit[m][h] <= start) continue;          // the row does not exist or sees none of the chunk
-        const int64_t state = qr * p.num_splits + chunk;
-        float2 *dst = reinterpret_cast<float2 *>(p.part_acc + state * 128 + 2 * t);
-#pragma unroll
-        for (int n = 0; n < 16; ++n) dst[4 * n] = make_float2(o[m][n][2 * h], o[m][n][2 * h + 1]);
-        if (t == 0) {
-          p.part_m[state] = mx[m][h];
-          p.part_l[state] = l;
-        }
-      }
+    __syncwarp();
+    tiles_all += nt;
+    tiles_m[0] += ntiles[0];
+    tiles_m[1] += ntiles[1];
   }
-  asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+  fence_before();
+  __syncthreads();
+  if (tid == 0 && lds32(kAbort) != 0u) {
+    p.work_counter[1] = (int)lds32(kAbort);                 // (for whoever looks into the workspace)
+    if (p.status) atomicOr(p.status, WTQ_STATUS_SCAN_TIMEOUT);
+  }
+  if (warp == kMmaWarp)
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(kCols) : "memory");
 }
 
 template <int BWK, int BWV>
