@@ -23,9 +23,12 @@
 //
 // Why tensor memory for A: an M 128, N 128, K 16 product with both operands in shared memory
 // reads 8 KB of it in its 64 cycles, all that the SM's shared memory delivers, and the
-// table lookups and the staging need as much again.  2^20 rows of 4 bits to bf16: 162 us with A
-// in shared memory, 109 us here; with the output stores left out 83, with the lookups left out
-// 107 (a plain fill of the output alone takes 73).
+// table lookups and the staging need as much again; and TMA stores, because plain ones back
+// up the load/store pipes that lookups, staging and tcgen05.ld go through.  2^20 rows of 4 bits
+// to bf16 (graph replay): 146 us with A in shared memory, 105 with A in tensor memory, 87 with
+// TMA stores, of which the products take 45 at 1965 MHz; a plain fill of the output takes 73.
+#include <cuda.h>
+
 #include <atomic>
 #include <mutex>
 
@@ -55,15 +58,17 @@ constexpr float kOperandScale = 256.f, kResultScale = 1.f / (256.f * 256.f);
 // instruction descriptor: dense, fp32 accumulator, fp16 A and B, both K-major, N = 128, M = 128
 constexpr uint32_t kIdesc = (1u << 4) | ((128u >> 3) << 17) | ((128u >> 4) << 24);
 
+constexpr uint32_t kBox = 32 * 128;
+
 template <int BW, int TERMS, int DT> struct Map {
   static constexpr uint32_t kLutBytes = mma::lut_entries(BW) * 256u;
   static constexpr uint32_t kBLo = mma::kLutAddr + kLutBytes;
-  // output staging: kPassRows rows of a warp's columns at a time, 16 bytes of padding per row
-  // (so that the rows of a pass land in different banks)
+  // output staging: boxes of 32 rows x 128 bytes in the 128-byte swizzle (piece k of row r lies
+  // at piece k ^ (r % 8)); a warp holds two: both of a tile (fp32), or of two tiles in turn
   static constexpr int kEsize = DT == WTQ_F32 ? 4 : 2;
-  static constexpr int kPassRows = kEsize == 2 ? 32 : 16;
-  static constexpr uint32_t kRowBytes = kWarpCols * kEsize, kStride = kRowBytes + 16;
-  static constexpr uint32_t kStage = kBLo + (TERMS == 3 ? kOperand : 0u), kStageBytes = kPassRows * kStride;
+  static constexpr int kBoxes = kWarpCols * kEsize / 128, kBoxCols = 128 / kEsize;
+  static constexpr uint32_t kStage = kBLo + (TERMS == 3 ? kOperand : 0u), kStageBytes = 2 * kBox;
+  static_assert(kStage % 1024 == 0, "swizzle atoms");
   static constexpr uint32_t kDynamic = kStage + kDrainWarps * kStageBytes;
   static_assert(kDynamic <= 227u * 1024u, "shared memory budget");
   // Table entries.  A 4-bit split table holds the high and the low pair of a byte's two codes
@@ -161,7 +166,8 @@ template <int DT> __device__ __forceinline__ uint32_t pack2(float x, float y) {
 // state: word 0 = 1 when the shared-memory layout assumption is broken, word 1 =
 // 1 when a wait for the tensor cores ran out.
 template <int BW, int TERMS, int DT>
-__global__ void __launch_bounds__(kThreads, 1) dequant_umma_kernel(DequantParams p, int32_t *state) {
+__global__ void __launch_bounds__(kThreads, 1)
+dequant_umma_kernel(DequantParams p, const __grid_constant__ CUtensorMap out_map, int32_t *state) {
   using M = Map<BW, TERMS, DT>;
   extern __shared__ __align__(128) uint8_t dyn_smem[];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -313,7 +319,7 @@ __global__ void __launch_bounds__(kThreads, 1) dequant_umma_kernel(DequantParams
     const int dw = warp - kFeedWarps, lr = 32 * (dw & 3) + lane;
     const uint32_t d_addr = tmem + ((uint32_t)(32 * (dw & 3)) << 16) + kColD + (uint32_t)(kWarpCols * (dw >> 2));
     const uint32_t stage = M::kStage + (uint32_t)dw * M::kStageBytes;
-    constexpr int kRowBytes = M::kRowBytes, kPassRows = M::kPassRows;
+    constexpr int kRowBytes = kWarpCols * M::kEsize;
     int64_t tile = blockIdx.x;
     __half nrm16 = __ushort_as_half(0);
     if (tile < tiles) nrm16 = p.norms[source_of(tile, lr)];
@@ -336,9 +342,11 @@ __global__ void __launch_bounds__(kThreads, 1) dequant_umma_kernel(DequantParams
       __syncwarp();
       if (lane == 0)
         asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(kBarFree + 8u * buf) : "memory");
-      // The thread holds consecutive columns of ONE row; stored as they are, every
-      // store instruction of the warp would touch 32 rows.  They go through a staging
-      // area instead and leave as whole row segments.
+      // The thread holds consecutive columns of ONE row; stored as they are, every store
+      // instruction of the warp would touch 32 rows.  They go through shared memory instead
+      // (the swizzle puts the eight lanes that store together into different banks) and leave
+      // as boxes by TMA, which keeps the stores out of the load/store pipes that the lookups,
+      // the staging and the tensor-memory loads share.
       uint32_t q[kRowBytes / 4];                            // the row segment, converted
 #pragma unroll
       for (int j = 0; j < kWarpCols / 32; ++j) {
@@ -351,29 +359,31 @@ __global__ void __launch_bounds__(kThreads, 1) dequant_umma_kernel(DequantParams
             q[16 * j + k] = pack2<DT>(__uint_as_float(v[j][2 * k]) * nrm, __uint_as_float(v[j][2 * k + 1]) * nrm);
         }
       }
-      uint8_t *base = (uint8_t *)p.out + (dw >> 2) * kRowBytes;
+      const uint32_t box = stage + (M::kBoxes == 1 ? (uint32_t)buf * kBox : 0u);
+      if (lane == 0) {                                       // the box written before is read out
+        if constexpr (M::kBoxes == 1) asm volatile("cp.async.bulk.wait_group.read 1;\n" ::: "memory");
+        else asm volatile("cp.async.bulk.wait_group.read 0;\n" ::: "memory");
+      }
+      __syncwarp();
+#pragma unroll
+      for (int k = 0; k < kRowBytes / 16; ++k)
+        sts128(box + (uint32_t)(k >> 3) * kBox + (uint32_t)lane * 128u + (uint32_t)((k & 7) ^ (lane & 7)) * 16u,
+               q[4 * k], q[4 * k + 1], q[4 * k + 2], q[4 * k + 3]);
+      asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+      __syncwarp();
       const int64_t n0 = (tile << 7) + 32 * (dw & 3);
+      if (lane == 0) {
+        if (n0 < p.N) {                                      // (rows past the end are clipped by the map)
 #pragma unroll
-      for (int ps = 0; ps < 32 / kPassRows; ++ps) {
-        if (kPassRows == 32 || lane / kPassRows == ps) {
-#pragma unroll
-          for (int k = 0; k < kRowBytes / 16; ++k)
-            sts128(stage + (uint32_t)(lane % kPassRows) * M::kStride + 16u * k, q[4 * k], q[4 * k + 1], q[4 * k + 2],
-                   q[4 * k + 3]);
+          for (int h = 0; h < M::kBoxes; ++h)
+            asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.tile.bulk_group [%0, {%1, %2}], [%3];\n"
+                         ::"l"(&out_map), "r"(kWarpCols * (dw >> 2) + M::kBoxCols * h), "r"((int)n0),
+                         "r"(box + (uint32_t)h * kBox) : "memory");
         }
-        __syncwarp();
-        constexpr int kPieces = kPassRows * kRowBytes / 16;
-        static_assert(kPieces % 32 == 0, "a pass is a whole number of warp-wide copies");
-#pragma unroll
-        for (int k = 0; k < kPieces / 32; ++k) {
-          const int c = lane + 32 * k, r = c / (kRowBytes / 16), piece = c % (kRowBytes / 16);
-          const uint4 x = lds128(stage + (uint32_t)r * M::kStride + 16u * piece);
-          const int64_t n = n0 + ps * kPassRows + r;
-          if (n < p.N) *reinterpret_cast<uint4 *>(base + n * (128 * M::kEsize) + 16 * piece) = x;
-        }
-        __syncwarp();
+        asm volatile("cp.async.bulk.commit_group;\n" ::: "memory");
       }
     }
+    if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;\n" ::: "memory");
   } else if (lane == 0) {
     // ---- multiply: one thread ----------------------------------------------------------------
     int i = 0;
@@ -421,6 +431,32 @@ template <int BW, int TERMS, int DT> std::atomic<int> &variant_state(int dev) {
 
 }  // namespace
 
+// Tensor map of an output, (N, 128) elements, boxes of 32 rows x 128 bytes; false where the
+// driver has no such call or refuses the tensor.
+template <int DT> static bool output_map(CUtensorMap *map, void *out, int64_t N) {
+  using Encode = CUresult (*)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
+                              const cuuint64_t *, const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave,
+                              CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+  static const Encode encode = [] {
+    void *f = nullptr;
+    cudaDriverEntryPointQueryResult found;
+    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &f, cudaEnableDefault, &found) != cudaSuccess ||
+        found != cudaDriverEntryPointSuccess)
+      f = nullptr;
+    return (Encode)f;
+  }();
+  if (!encode || N >= (int64_t)1 << 31) return false;
+  constexpr int kEsize = DT == WTQ_F32 ? 4 : 2;
+  const cuuint64_t dims[2] = {128, (cuuint64_t)N}, strides[1] = {128 * kEsize};
+  const cuuint32_t box[2] = {128 / kEsize, 32}, steps[2] = {1, 1};
+  const CUtensorMapDataType type = DT == WTQ_F32   ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32
+                                   : DT == WTQ_F16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16
+                                                   : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
+  return encode(map, type, 2, out, dims, strides, box, steps, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_NONE,
+                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
 // Runs the tcgen05 kernel.  `*usable` comes back false (and nothing was
 // launched for the call) when the kernel cannot be used here: the stream is
 // capturing and the variant has not been set up yet, or the device places
@@ -451,7 +487,7 @@ static int launch_variant(const DequantParams &p, cudaStream_t stream, bool *usa
       if (e == cudaSuccess) {
         DequantParams none = {};
         none.L = none.MAXLEN = 1;
-        kernel<<<1, dq5::kThreads, M::kDynamic, stream>>>(none, flag);
+        kernel<<<1, dq5::kThreads, M::kDynamic, stream>>>(none, CUtensorMap{}, flag);
         note_launches(1);
         e = cudaGetLastError();
       }
@@ -465,7 +501,9 @@ static int launch_variant(const DequantParams &p, cudaStream_t stream, bool *usa
   if (s != 1) return WTQ_OK;
   const int64_t tiles = (p.N + 127) / 128;
   const int grid = (int)std::min<int64_t>(tiles, device_sms());
-  kernel<<<grid, dq5::kThreads, M::kDynamic, stream>>>(p, flag);
+  CUtensorMap map;
+  if (!output_map<DT>(&map, p.out, p.N)) return WTQ_OK;
+  kernel<<<grid, dq5::kThreads, M::kDynamic, stream>>>(p, map, flag);
   note_launches(1);
   *usable = true;
   return check_cuda(cudaGetLastError(), "wtq_dequant tensor-memory launch");
