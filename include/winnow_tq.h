@@ -306,6 +306,12 @@ int wtq_dequant(const uint8_t *packed, const void *norms_f16, const float *centr
 int wtq_dequant_mode(const uint8_t *packed, const void *norms_f16, const float *centroids,
                      const float *Pi, void *out, int out_dtype, int bw, int D, int64_t N, int64_t L,
                      int64_t MAXLEN, int mode, void *stream);
+/* wtq_dequant of two tensors of one shape, width and quantizer (K and V of a layer), each
+ * with its own packed rows, norms and output: the same results in one launch where the
+ * tcgen05 kernel applies. */
+int wtq_dequant_pair(const uint8_t *const packed[2], const void *const norms_f16[2],
+                     const float *centroids, const float *Pi, void *const out[2], int out_dtype,
+                     int bw, int D, int64_t N, int64_t L, int64_t MAXLEN, void *stream);
 
 /* Instrumentation; no counterpart in the reference.
  * wtq_launch_count: kernels this library has launched in this process.

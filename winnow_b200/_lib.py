@@ -104,6 +104,9 @@ _SIGNATURES = {
                             c_int64, c_int64, c_int64, c_void_p]),
     "wtq_dequant_mode": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int,
                                  c_int, c_int64, c_int64, c_int64, c_int, c_void_p]),
+    "wtq_dequant_pair": (c_int, [ctypes.POINTER(c_void_p), ctypes.POINTER(c_void_p), c_void_p, c_void_p,
+                                 ctypes.POINTER(c_void_p), c_int, c_int, c_int, c_int64, c_int64, c_int64,
+                                 c_void_p]),
 }
 
 _lib = None

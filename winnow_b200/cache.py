@@ -8,6 +8,7 @@ on the GPU through libwinnow_tq.
 """
 from __future__ import annotations
 
+import ctypes
 import math
 
 import numpy as np
@@ -311,6 +312,23 @@ class TQPackedLayer(_LayerBase):
             out.index_copy_(-1, channels, part)
         return out
 
+    def _load_both(self, length):
+        """`_load` of K and of V; without outlier channels in one launch."""
+        if self._out_dim or not length:
+            return self._load(length, self._k), self._load(length, self._v)
+        B, H, D = self._shape
+        outs = [torch.empty(B, H, length, D, dtype=self.dtype, device=self.device) for _ in range(2)]
+        if B * H:
+            pair = ctypes.c_void_p * 2
+            with torch.cuda.device(self.device):
+                _lib.check(_lib.lib().wtq_dequant_pair(
+                    pair(self._k[0].data_ptr(), self._v[0].data_ptr()),
+                    pair(self._k[1].data_ptr(), self._v[1].data_ptr()),
+                    self._tq.centroids.data_ptr(), self._tq.Pi.data_ptr(),
+                    pair(outs[0].data_ptr(), outs[1].data_ptr()), _lib.dtype_code(self.dtype), self._bw, D,
+                    B * H * length, length, self._max, _lib.stream_ptr(self.device)))
+        return outs[0], outs[1]
+
     @torch.no_grad()
     def update(self, key_states, value_states, *args, **kwargs):
         if not self.is_initialized:
@@ -323,7 +341,7 @@ class TQPackedLayer(_LayerBase):
             self._store(key_states, self._len, n, self._k)
             self._store(value_states, self._len, n, self._v)
         self._len += n
-        return self._load(self._len, self._k), self._load(self._len, self._v)
+        return self._load_both(self._len)
 
     # ---- cache protocol ----------------------------------------------------------
     def get_seq_length(self, *args, **kwargs) -> int:

@@ -12,6 +12,11 @@ struct DequantParams {
   void *out;
   int out_dtype, bw, D, nb;
   int64_t N, L, MAXLEN;
+  // a second tensor of the same shape, widths and quantizer (tcgen05 kernel only)
+  int tensors = 1;
+  const uint8_t *packed_b = nullptr;
+  const __half *norms_b = nullptr;
+  void *out_b = nullptr;
 };
 
 // tcgen05 kernel (wtq_dequant_umma.cu); `terms` = 1 or 3.  *usable = false and

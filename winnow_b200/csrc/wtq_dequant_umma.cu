@@ -167,7 +167,8 @@ template <int DT> __device__ __forceinline__ uint32_t pack2(float x, float y) {
 // 1 when a wait for the tensor cores ran out.
 template <int BW, int TERMS, int DT>
 __global__ void __launch_bounds__(kThreads, 1)
-dequant_umma_kernel(DequantParams p, const __grid_constant__ CUtensorMap out_map, int32_t *state) {
+dequant_umma_kernel(DequantParams p, const __grid_constant__ CUtensorMap out_map,
+                    const __grid_constant__ CUtensorMap out_map_b, int32_t *state) {
   using M = Map<BW, TERMS, DT>;
   extern __shared__ __align__(128) uint8_t dyn_smem[];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -236,11 +237,17 @@ dequant_umma_kernel(DequantParams p, const __grid_constant__ CUtensorMap out_map
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
   const uint32_t tmem = lds32(kTmemSlot);
+  // The set-up above read the codebook and Pi only (which no kernel that lets its successor
+  // in early writes) and ran under the tail of the kernel ahead; codes, norms and outputs are
+  // touched after all earlier kernels.  The next kernel's blocks may move in as ours leave.
+  asm volatile("griddepcontrol.wait;\n" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
 
-  const int64_t tiles = (p.N + 127) >> 7;
+  // a call over two tensors (K and V of a layer): the second one's tiles follow the first's
+  const int64_t tiles_each = (p.N + 127) >> 7, tiles = tiles_each * p.tensors;
   const uint32_t L32 = (uint32_t)p.L;
   const bool dense = p.L == p.MAXLEN;                       // source row = logical row: no plane arithmetic
-  // source row of row lr of a tile (rows past the end re-read the last one)
+  // source row of row lr of a tile of one tensor (rows past the end re-read the last one)
   auto source_of = [&](int64_t tile, int lr) -> int64_t {
     const int64_t row0 = tile << 7;
     lr = min(lr, (int)min((int64_t)127, p.N - 1 - row0));
@@ -276,7 +283,9 @@ dequant_umma_kernel(DequantParams p, const __grid_constant__ CUtensorMap out_map
     const uint32_t sel = mma::kLutAddr | (uint32_t)(lane << M::kLaneShift);
     const uint32_t a_addr = tmem + ((uint32_t)(32 * (warp & 3)) << 16) + kColA + 32u * half;
     auto fetch = [&](int64_t tile, uint32_t (&w)[2 * BW]) {
-      load_half<BW>(p.packed + source_of(tile, lr) * (16 * BW) + half * (8 * BW), w);
+      const bool second = tile >= tiles_each;
+      load_half<BW>((second ? p.packed_b : p.packed) + source_of(tile - (second ? tiles_each : 0), lr) * (16 * BW) +
+                        half * (8 * BW), w);
     };
     // one tile: codes in w to operand buf; then w is refilled for the tile after next
     auto feed = [&](int64_t tile, int i, int buf, uint32_t (&w)[2 * BW]) -> bool {
@@ -321,12 +330,16 @@ dequant_umma_kernel(DequantParams p, const __grid_constant__ CUtensorMap out_map
     const uint32_t stage = M::kStage + (uint32_t)dw * M::kStageBytes;
     constexpr int kRowBytes = kWarpCols * M::kEsize;
     int64_t tile = blockIdx.x;
+    auto norm_at = [&](int64_t at) {
+      const bool second = at >= tiles_each;
+      return (second ? p.norms_b : p.norms)[source_of(at - (second ? tiles_each : 0), lr)];
+    };
     __half nrm16 = __ushort_as_half(0);
-    if (tile < tiles) nrm16 = p.norms[source_of(tile, lr)];
+    if (tile < tiles) nrm16 = norm_at(tile);
     for (int i = 0; tile < tiles; tile += gridDim.x, ++i) {
       const int buf = i & 1;
       const float nrm = __half2float(nrm16) * kResultScale;
-      if (tile + gridDim.x < tiles) nrm16 = p.norms[source_of(tile + gridDim.x, lr)];
+      if (tile + gridDim.x < tiles) nrm16 = norm_at(tile + gridDim.x);
       const bool ok = wait_for(kBarDone + 8u * buf, i >> 1);
       if (!__all_sync(0xffffffffu, ok)) {
         if (lane == 0) state[1] = 1;
@@ -371,13 +384,14 @@ dequant_umma_kernel(DequantParams p, const __grid_constant__ CUtensorMap out_map
                q[4 * k], q[4 * k + 1], q[4 * k + 2], q[4 * k + 3]);
       asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
       __syncwarp();
-      const int64_t n0 = (tile << 7) + 32 * (dw & 3);
+      const bool second = tile >= tiles_each;
+      const int64_t n0 = ((tile - (second ? tiles_each : 0)) << 7) + 32 * (dw & 3);
       if (lane == 0) {
         if (n0 < p.N) {                                      // (rows past the end are clipped by the map)
 #pragma unroll
           for (int h = 0; h < M::kBoxes; ++h)
             asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.tile.bulk_group [%0, {%1, %2}], [%3];\n"
-                         ::"l"(&out_map), "r"(kWarpCols * (dw >> 2) + M::kBoxCols * h), "r"((int)n0),
+                         ::"l"(second ? &out_map_b : &out_map), "r"(kWarpCols * (dw >> 2) + M::kBoxCols * h), "r"((int)n0),
                          "r"(box + (uint32_t)h * kBox) : "memory");
         }
         asm volatile("cp.async.bulk.commit_group;\n" ::: "memory");
@@ -487,7 +501,7 @@ static int launch_variant(const DequantParams &p, cudaStream_t stream, bool *usa
       if (e == cudaSuccess) {
         DequantParams none = {};
         none.L = none.MAXLEN = 1;
-        kernel<<<1, dq5::kThreads, M::kDynamic, stream>>>(none, CUtensorMap{}, flag);
+        kernel<<<1, dq5::kThreads, M::kDynamic, stream>>>(none, CUtensorMap{}, CUtensorMap{}, flag);
         note_launches(1);
         e = cudaGetLastError();
       }
@@ -499,14 +513,25 @@ static int launch_variant(const DequantParams &p, cudaStream_t stream, bool *usa
     }
   }
   if (s != 1) return WTQ_OK;
-  const int64_t tiles = (p.N + 127) / 128;
+  const int64_t tiles = (p.N + 127) / 128 * p.tensors;
   const int grid = (int)std::min<int64_t>(tiles, device_sms());
-  CUtensorMap map;
-  if (!output_map<DT>(&map, p.out, p.N)) return WTQ_OK;
-  kernel<<<grid, dq5::kThreads, M::kDynamic, stream>>>(p, map, flag);
+  CUtensorMap map, map_b;
+  if (!output_map<DT>(&map, p.out, p.N) || !output_map<DT>(&map_b, p.tensors == 2 ? p.out_b : p.out, p.N))
+    return WTQ_OK;
+  cudaLaunchAttribute pdl;
+  pdl.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  pdl.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)grid);
+  cfg.blockDim = dim3(dq5::kThreads);
+  cfg.dynamicSmemBytes = M::kDynamic;
+  cfg.stream = stream;
+  cfg.attrs = &pdl;
+  cfg.numAttrs = 1;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, p, map, map_b, flag);
   note_launches(1);
   *usable = true;
-  return check_cuda(cudaGetLastError(), "wtq_dequant tensor-memory launch");
+  return check_cuda(e, "wtq_dequant tensor-memory launch");
 }
 
 template <int BW, int TERMS>
