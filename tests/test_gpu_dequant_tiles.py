@@ -39,3 +39,28 @@ def test_two_tensors_are_two_calls(planes, length, maxlen, bw, dtype, D):
         dequantize_rows(codes[:, :length], norms[:, :length], tq.centroids, tq.Pi, bw, D, out=one)
         assert torch.equal(out, one.view(N, D))
         assert (guard[:32] == -12352.0).all() and (guard[32 + N:] == -12352.0).all()
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("bw", [2, 3, 4, 5, 6, 8])
+@pytest.mark.parametrize("planes,length,maxlen", [(1, 1, 1), (1, 129, 129), (3, 85, 90), (1, 257, 300)])
+def test_fp32_register_tiles(D, bw, planes, length, maxlen):
+    """Sums of D products in fp32: the kernel's chain and the oracle's differ by at most
+    2 D 2^-24 of the sum of the products' magnitudes, which is at most |y| |Pi column| = |y|
+    <= sqrt(D) times the largest centroid (Pi is orthogonal)."""
+    tq = _get_quantizer(bw, D, DEV, 42)
+    codes, norms = _rows(planes, maxlen, D, bw, 7)
+    N = planes * length
+    for dtype in (torch.float32, torch.bfloat16):
+        guard = torch.full((N + 64, D), -12352.0, dtype=dtype, device=DEV)
+        out = guard[32:32 + N].view(planes, length, D)
+        dequantize_rows(codes.to(DEV)[:, :length], norms.to(DEV)[:, :length], tq.centroids, tq.Pi, bw, D, out=out,
+                        mode="exact")
+        o = orc.OracleQuantizer.get(bw, D, 42)
+        ref = orc.dequantize_rows(codes[:, :length].contiguous(), norms[:, :length].contiguous(), o.centroids, o.Pi,
+                                  bw, D)
+        bound = 2 * D * 2.0 ** -24 * D ** 0.5 * float(o.centroids.abs().max()) * norms[:, :length, None].float()
+        if dtype == torch.bfloat16:
+            bound = bound + ref.abs() * 2.0 ** -8
+        assert ((out.float().cpu() - ref.reshape(out.shape)).abs() <= bound).all()
+        assert (guard[:32] == -12352.0).all() and (guard[32 + N:] == -12352.0).all()
