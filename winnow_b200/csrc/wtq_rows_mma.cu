@@ -7,14 +7,19 @@
 //   merge   out[r][c]   = sum_d a[r][d] Pi[d][c],  a = merged and normalised
 //           chunk states of row r (the arithmetic of merge_small_kernel)
 //
-// A warp takes 32 rows.  The A fragments of mma.m16n8k16 are made in registers
-// from global loads (two adjacent coordinates per register), each value split
-// into fp16 high and low parts; the rotation sits in shared memory as fp16 high
-// and low parts times 2^8, one row per output coordinate, fetched with
-// ldmatrix; the three significant products accumulate in fp32 (the dropped
-// low x low term is 2^-22 of a product).  The epilogue turns the fragment layout
-// into whole 256-byte row segments through a per-warp staging area, as the
-// dequantisation kernel does.
+// A warp takes 32 rows.  It reads them whole, sixteen loads of a row each in
+// flight (merge: per chunk, predicated on the chunk's weight), and puts them into
+// its part of shared memory as fp16 high and low parts; the rotation sits in shared
+// memory as fp16 high and low parts times 2^8, one row per output coordinate; both
+// are fetched with ldmatrix and the three significant products accumulate in fp32
+// (the dropped low x low term is 2^-22 of a product).  The epilogue turns the
+// fragment layout into whole 256-byte row segments through a per-warp staging area,
+// as the dequantisation kernel does.
+//
+// Bound: latency (a warp has one tile of a call of 32 K rows).  With the fragments
+// loaded pair by pair behind a branch per chunk the loads came one after another:
+// 32 K rows with up to three chunks 71 us for the merge and 22 for the rotation, 21 and 15 now
+// (of which the products are 7).
 #include <algorithm>
 #include <atomic>
 
@@ -29,11 +34,13 @@ constexpr uint32_t kBase = 1024;                  // dynamic shared memory is as
 constexpr uint32_t kPiRow = 272;                  // 256 + 16: ldmatrix conflict-free
 constexpr uint32_t kPiBytes = 128 * kPiRow;
 constexpr uint32_t kPiHi = kBase, kPiLo = kPiHi + kPiBytes;
-constexpr uint32_t kStage = kPiLo + kPiBytes;
-constexpr uint32_t kStageBytes = 16 * 288;        // per warp: 16 rows x 256 payload bytes (+ pad)
-constexpr uint32_t kWeights = kStage + kWarps * kStageBytes;   // merge: 32 rows x kMaxChunks weights per warp
+constexpr uint32_t kRowsHi = kPiLo + kPiBytes;    // per warp: 32 rows, high parts then low parts
+constexpr uint32_t kPartBytes = 32 * kPiRow, kRowsBytes = 2 * kPartBytes;
+static_assert(16 * 288 <= kRowsBytes, "the output staging area (16 rows x 256 payload bytes + pad) reuses the rows");
+constexpr uint32_t kWeights = kRowsHi + kWarps * kRowsBytes;   // merge: 32 rows x kMaxChunks weights per warp
 constexpr int kMaxChunks = 8;
 constexpr uint32_t kDynamic = kWeights + kWarps * 32 * kMaxChunks * 4;
+static_assert(kDynamic <= 227u * 1024u, "shared memory budget");
 constexpr float kPiScale = 256.f;
 
 struct Params {
@@ -63,6 +70,20 @@ __device__ __forceinline__ void ldmatrix_x4(uint32_t a, uint32_t (&r)[4]) {
 }
 __device__ __forceinline__ void sts64f(uint32_t a, float x, float y) {
   asm volatile("st.shared.v2.f32 [%0], {%1,%2};\n" ::"r"(a), "f"(x), "f"(y) : "memory");
+}
+__device__ __forceinline__ void sts64(uint32_t a, uint32_t x, uint32_t y) {
+  asm volatile("st.shared.v2.u32 [%0], {%1,%2};\n" ::"r"(a), "r"(x), "r"(y) : "memory");
+}
+// 16 bytes, or zeros without an access where w is 0 (a predicate, not a branch: the loads of
+// several rows stay together)
+__device__ __forceinline__ float4 load_if(float w, const float *at) {
+  float4 v;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tsetp.neu.f32 p, %4, 0f00000000;\n\t"
+      "mov.f32 %0, 0f00000000;\n\tmov.f32 %1, 0f00000000;\n\tmov.f32 %2, 0f00000000;\n\tmov.f32 %3, 0f00000000;\n\t"
+      "@p ld.global.cg.v4.f32 {%0, %1, %2, %3}, [%5];\n\t}\n"
+      : "=&f"(v.x), "=&f"(v.y), "=&f"(v.z), "=&f"(v.w) : "f"(w), "l"(at) : "memory");
+  return v;
 }
 template <int DT> __device__ __forceinline__ uint32_t pack2(float x, float y) {
   if constexpr (DT == WTQ_BF16) {
@@ -123,16 +144,17 @@ __global__ void __launch_bounds__(kThreads, 1) rows_kernel(Params p) {
   if constexpr (MERGE) asm volatile("griddepcontrol.wait;\n" ::: "memory");   // chunk states are complete
 
   const uint32_t lane_off = (uint32_t)(((lane >> 4) * 8 + (lane & 7)) * kPiRow + ((lane >> 3) & 1) * 16);
-  const uint32_t stage = kStage + (uint32_t)warp * kStageBytes;
+  const uint32_t rows_hi = kRowsHi + (uint32_t)warp * kRowsBytes, rows_lo = rows_hi + kPartBytes, stage = rows_hi;
+  const uint32_t a_off = (uint32_t)((lane & 15) * kPiRow + (lane >> 4) * 16);
   const uint32_t weights = kWeights + (uint32_t)warp * (32 * kMaxChunks * 4);
   const int64_t tiles = (p.rows + 31) >> 5;
   constexpr int kEsize = DT == WTQ_F32 ? 4 : 2;
   constexpr uint32_t kStageRow = kEsize == 4 ? 288u : 272u;
 
-  for (int64_t tile = (int64_t)blockIdx.x * kWarps + warp; tile < tiles; tile += (int64_t)gridDim.x * kWarps) {
+  for (int64_t tile = blockIdx.x + (int64_t)gridDim.x * warp; tile < tiles; tile += (int64_t)gridDim.x * kWarps) {
     const int64_t row0 = tile << 5;
     // ---- merge: lane l computes the chunk weights of row row0 + l -----------------
-    int chunks_of[2][2] = {{0, 0}, {0, 0}};
+    int most = 0;                                            // chunks of the row that has most
     if constexpr (MERGE) {
       const int64_t row = row0 + lane;
       int chunks = 0;
@@ -159,42 +181,69 @@ __global__ void __launch_bounds__(kThreads, 1) rows_kernel(Params p) {
 #pragma unroll
       for (int c = 0; c < kMaxChunks; ++c) sts32(weights + (uint32_t)(lane * kMaxChunks + c) * 4u, __float_as_uint(mv[c] * inv));
       __syncwarp();
-#pragma unroll
-      for (int m = 0; m < 2; ++m)
-#pragma unroll
-        for (int h = 0; h < 2; ++h) chunks_of[m][h] = __shfl_sync(0xffffffffu, chunks, 16 * m + 8 * h + g);
+      most = __reduce_max_sync(0xffffffffu, chunks);
     }
-    // values (d, d + 1) of the lane's row (m, h), d even
-    auto pair_at = [&](int m, int h, int d) -> float2 {
-      const int lr = 16 * m + 8 * h + g;
-      const int64_t row = row0 + lr;
-      if (row >= p.rows) return make_float2(0.f, 0.f);
-      if constexpr (!MERGE) {
-        if (p.in_dtype == WTQ_F32) {
-          return __ldg(reinterpret_cast<const float2 *>((const float *)p.q + row * 128 + d));
-        } else if (p.in_dtype == WTQ_F16) {
-          return __half22float2(__ldg(reinterpret_cast<const __half2 *>((const __half *)p.q + row * 128 + d)));
-        } else {
-          return __bfloat1622float2(
-              __ldg(reinterpret_cast<const __nv_bfloat162 *>((const __nv_bfloat16 *)p.q + row * 128 + d)));
-        }
-      } else {
-        float2 a = make_float2(0.f, 0.f);
-        const float *src = p.part_acc + row * p.num_splits * 128 + d;
+    // ---- the rows into shared memory, a whole row per warp-wide load -------------------
+    constexpr int kBatch = 16;
+#pragma unroll 1
+    for (int r0 = 0; r0 < 32; r0 += kBatch) {
+      float4 a[kBatch];
+      if constexpr (MERGE) {
 #pragma unroll
-        for (int c = 0; c < kMaxChunks; ++c) {
-          if (c < chunks_of[m][h]) {
-            const float w = __uint_as_float(lds32(weights + (uint32_t)(lr * kMaxChunks + c) * 4u));
-            if (w != 0.f) {
-              const float2 v = __ldcg(reinterpret_cast<const float2 *>(src + c * 128));
-              a.x = fmaf(w, v.x, a.x);
-              a.y = fmaf(w, v.y, a.y);
-            }
+        for (int r = 0; r < kBatch; ++r) a[r] = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 1
+        for (int c = 0; c < most; ++c) {
+          float w[kBatch];
+          float4 v[kBatch];
+          const float *src = p.part_acc + ((row0 + r0) * p.num_splits + c) * 128 + 4 * lane;
+#pragma unroll
+          for (int r = 0; r < kBatch; ++r) w[r] = __uint_as_float(lds32(weights + (uint32_t)((r0 + r) * kMaxChunks + c) * 4u));
+#pragma unroll
+          for (int r = 0; r < kBatch; ++r) v[r] = load_if(w[r], src + (int64_t)r * p.num_splits * 128);
+#pragma unroll
+          for (int r = 0; r < kBatch; ++r) {
+            a[r].x = fmaf(w[r], v[r].x, a[r].x);
+            a[r].y = fmaf(w[r], v[r].y, a[r].y);
+            a[r].z = fmaf(w[r], v[r].z, a[r].z);
+            a[r].w = fmaf(w[r], v[r].w, a[r].w);
           }
         }
-        return a;
+      } else if (p.in_dtype == WTQ_F32) {
+#pragma unroll
+        for (int r = 0; r < kBatch; ++r)
+          a[r] = row0 + r0 + r < p.rows
+                     ? __ldg(reinterpret_cast<const float4 *>((const float *)p.q + (row0 + r0 + r) * 128) + lane)
+                     : make_float4(0.f, 0.f, 0.f, 0.f);
+      } else {
+        uint2 v[kBatch];
+#pragma unroll
+        for (int r = 0; r < kBatch; ++r)
+          v[r] = row0 + r0 + r < p.rows
+                     ? __ldg(reinterpret_cast<const uint2 *>((const uint16_t *)p.q + (row0 + r0 + r) * 128) + lane)
+                     : make_uint2(0u, 0u);
+#pragma unroll
+        for (int r = 0; r < kBatch; ++r) {
+          float2 x, y;
+          if (p.in_dtype == WTQ_F16) {
+            x = __half22float2(*reinterpret_cast<const __half2 *>(&v[r].x));
+            y = __half22float2(*reinterpret_cast<const __half2 *>(&v[r].y));
+          } else {
+            x = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162 *>(&v[r].x));
+            y = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162 *>(&v[r].y));
+          }
+          a[r] = make_float4(x.x, x.y, y.x, y.y);
+        }
       }
-    };
+#pragma unroll
+      for (int r = 0; r < kBatch; ++r) {
+        uint32_t h0, l0, h1, l1;
+        split(a[r].x, a[r].y, h0, l0);
+        split(a[r].z, a[r].w, h1, l1);
+        sts64(rows_hi + (uint32_t)(r0 + r) * kPiRow + 8u * lane, h0, h1);
+        sts64(rows_lo + (uint32_t)(r0 + r) * kPiRow + 8u * lane, l0, l1);
+      }
+    }
+    __syncwarp();
 
     float acc[2][16][4];
 #pragma unroll
@@ -208,12 +257,8 @@ __global__ void __launch_bounds__(kThreads, 1) rows_kernel(Params p) {
       uint32_t ah[2][4], al[2][4];
 #pragma unroll
       for (int m = 0; m < 2; ++m) {
-        const float2 v0 = pair_at(m, 0, 16 * ks + 2 * t), v1 = pair_at(m, 1, 16 * ks + 2 * t);
-        const float2 v2 = pair_at(m, 0, 16 * ks + 8 + 2 * t), v3 = pair_at(m, 1, 16 * ks + 8 + 2 * t);
-        split(v0.x, v0.y, ah[m][0], al[m][0]);
-        split(v1.x, v1.y, ah[m][1], al[m][1]);
-        split(v2.x, v2.y, ah[m][2], al[m][2]);
-        split(v3.x, v3.y, ah[m][3], al[m][3]);
+        ldmatrix_x4(rows_hi + a_off + m * 16 * kPiRow + ks * 32, ah[m]);
+        ldmatrix_x4(rows_lo + a_off + m * 16 * kPiRow + ks * 32, al[m]);
       }
 #pragma unroll
       for (int np = 0; np < 8; ++np) {
@@ -233,6 +278,7 @@ __global__ void __launch_bounds__(kThreads, 1) rows_kernel(Params p) {
     }
 
     // ---- epilogue: 16 rows x 256 payload bytes per pass through the staging area
+    __syncwarp();                                            // all lanes have read the rows it reuses
     const float post = (MERGE ? 1.f : p.mult) / kPiScale;
     constexpr int kPasses = kEsize == 4 ? 2 : 1;
 #pragma unroll
@@ -281,7 +327,7 @@ int launch(const Params &p, bool pdl, cudaStream_t stream) {
     opted_in_dev[dev & 63].store(true, std::memory_order_release);
   }
   const int64_t tiles = (p.rows + 31) / 32;
-  const int grid = (int)std::min<int64_t>((tiles + kWarps - 1) / kWarps, device_sms());
+  const int grid = (int)std::min<int64_t>(tiles, device_sms());    // tiles go to the blocks before their warps
   cudaLaunchAttribute attr;
   attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr.val.programmaticStreamSerializationAllowed = 1;
