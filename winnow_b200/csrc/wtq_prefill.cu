@@ -148,6 +148,12 @@ __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
 __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(bar) : "memory");
 }
+// 1 in one lane of a converged warp, the same every time
+__device__ __forceinline__ uint32_t elect_one() {
+  uint32_t r;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}\n" : "=r"(r));
+  return r;
+}
 // Bounded wait for completion number `use` (0, 1, ..) of an mbarrier; false if it, or any
 // other wait of the block, ran out.
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, int use) {
@@ -695,46 +701,64 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_kernel(Params p) {
           nrm[h] = nrm_next[h];
         }
       }
-    } else if (lane == 0) {
-      // ================= multiply: one thread ============================================
-      bool ok = true;
-      for (int j = 0; j <= nt && ok; ++j) {
+    } else {
+      // ================= multiply: the whole warp waits, one lane issues ======================
+      // (Control flow stays uniform and the two M tiles are spelled out: with one lane in the
+      // loop and the tile counts indexed, the code between the products took longer than
+      // the products and was what everybody waited for.)
+      const uint32_t issuer = elect_one();
+      const uint64_t q_desc = desc_k_major(M::kQTile, 0);
+      auto scores = [&](int j, auto m_) -> bool {                       // S of tile j, M tile m
+        constexpr int m = decltype(m_)::value;
+        const int T = tiles_all + j, buf = T & 1, Tm = tiles_m[m] + j, sb = Tm & 1;
+        // the buffer's last probabilities have been consumed (those of an earlier item were
+        // before its states were written)
+        if (j >= 2 && !mbar_wait(kODone + 16u * m + 8u * sb, (Tm - 2) >> 1)) return false;
+        fence_after();
+        if (issuer) {
+          const uint32_t d = tmem + kColS + 128u * m + 64u * sb;
+          const uint64_t qa = q_desc + (uint64_t)m * (32768u >> 4);
+          const uint64_t kb = desc_k_major(M::kKTile + (uint32_t)buf * kTileBytes, 0);
+#pragma unroll
+          for (int ks = 0; ks < 8; ++ks)
+            umma_ss(d, qa + 16u * ks, kb + 16u * ks, kIdescQK, ks > 0);
+          umma_commit(kSFull + 16u * m + 8u * sb);
+        }
+        return true;
+      };
+      auto values = [&](int i, auto m_) -> bool {                       // O += P V of tile i, M tile m
+        constexpr int m = decltype(m_)::value;
+        const int T = tiles_all + i, buf = T & 1, Tm = tiles_m[m] + i, sb = Tm & 1;
+        if (!mbar_wait(kPFull + 16u * m + 8u * sb, Tm >> 1)) return false;
+        fence_after();
+        if (issuer) {
+          const uint32_t p_addr = tmem + kColS + 128u * m + 64u * sb, d = tmem + kColO + 128u * m;
+          const uint64_t vb = desc_mn_major(kVTile + (uint32_t)buf * kTileBytes, 0);
+#pragma unroll
+          for (int ks = 0; ks < 4; ++ks)
+            umma_ts(d, p_addr + 8u * ks, vb + 256u * ks, kIdescPV, i > 0 || ks > 0);
+          umma_commit(kODone + 16u * m + 8u * sb);
+        }
+        return true;
+      };
+      constexpr std::integral_constant<int, 0> m0{};
+      constexpr std::integral_constant<int, 1> m1{};
+      for (int j = 0; j <= nt; ++j) {
         if (j < nt) {                                                   // scores of tile j
           const int T = tiles_all + j, buf = T & 1;
-          ok = mbar_wait(kKFull + 8u * buf, T >> 1);
-          for (int m = 0; m < 2 && ok; ++m) {
-            if (j >= ntiles[m]) continue;
-            const int Tm = tiles_m[m] + j, sb = Tm & 1;
-            // the buffer's last probabilities have been consumed (those of an earlier item were
-            // before its states were written)
-            if (j >= 2) ok = mbar_wait(kODone + 16u * m + 8u * sb, (Tm - 2) >> 1);
-            if (!ok) break;
-            fence_after();
-            const uint32_t d = tmem + kColS + 128u * m + 64u * sb;
-#pragma unroll
-            for (int ks = 0; ks < 8; ++ks)
-              umma_ss(d, desc_k_major(M::kQTile + (uint32_t)m * 32768u, ks),
-                      desc_k_major(M::kKTile + (uint32_t)buf * kTileBytes, ks), kIdescQK, ks > 0);
-            umma_commit(kSFull + 16u * m + 8u * sb);
-          }
-          if (ok) umma_commit(kKFree + 8u * buf);
+          bool ok = mbar_wait(kKFull + 8u * buf, T >> 1);
+          if (ok && j < ntiles[0]) ok = scores(j, m0);
+          if (ok && j < ntiles[1]) ok = scores(j, m1);
+          if (!__all_sync(kFull, ok)) break;
+          if (issuer) umma_commit(kKFree + 8u * buf);
         }
-        if (j > 0 && ok) {                                              // values of tile j - 1
-          const int i = j - 1, T = tiles_all + i, buf = T & 1;
-          ok = mbar_wait(kVFull + 8u * buf, T >> 1);
-          for (int m = 0; m < 2 && ok; ++m) {
-            if (i >= ntiles[m]) continue;
-            const int Tm = tiles_m[m] + i;
-            ok = mbar_wait(kPFull + 16u * m + 8u * (Tm & 1), Tm >> 1);
-            if (!ok) break;
-            fence_after();
-            const uint32_t a = tmem + kColS + 128u * m + 64u * (Tm & 1), d = tmem + kColO + 128u * m;
-#pragma unroll
-            for (int ks = 0; ks < 4; ++ks)
-              umma_ts(d, a + 8u * ks, desc_mn_major(kVTile + (uint32_t)buf * kTileBytes, ks), kIdescPV, i > 0 || ks > 0);
-            umma_commit(kODone + 16u * m + 8u * (Tm & 1));
-          }
-          if (ok) umma_commit(kVFree + 8u * buf);
+        if (j > 0) {                                                    // values of tile j - 1
+          const int T = tiles_all + j - 1, buf = T & 1;
+          bool ok = mbar_wait(kVFull + 8u * buf, T >> 1);
+          if (ok && j - 1 < ntiles[0]) ok = values(j - 1, m0);
+          if (ok && j - 1 < ntiles[1]) ok = values(j - 1, m1);
+          if (!__all_sync(kFull, ok)) break;
+          if (issuer) umma_commit(kVFree + 8u * buf);
         }
       }
     }
