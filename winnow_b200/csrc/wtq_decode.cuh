@@ -102,7 +102,8 @@ int launch_decode_fused(const DecodeParams &p, const void *q, int dtype, const i
 bool rows_mma_rotate_eligible(const void *q, int64_t row_stride, int64_t head_stride, int Hq, int D,
                               int64_t rows, const float *Pi, const float *q_rot);
 int launch_rotate_rows_mma(const void *q, int dtype, const float *Pi, float mult, int64_t rows,
-                           float *q_rot, const ScanSetup &setup, int32_t *status, cudaStream_t stream);
+                           float *q_rot, const ScanSetup &setup, float *zero, int64_t zero_words,
+                           int32_t *counter, int32_t *status, cudaStream_t stream);
 bool rows_mma_merge_eligible(const MergeParams &m, int64_t rows);
 int launch_merge_rows_mma(const MergeParams &m, const int32_t *row_lens, int64_t rows, int chunk_tokens,
                           int max_tokens, int32_t *status, cudaStream_t stream);

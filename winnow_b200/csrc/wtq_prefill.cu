@@ -956,22 +956,24 @@ extern "C" int wtq_prefill(const void *q, int dtype, const int64_t q_strides[2],
     return fail(WTQ_ERR_UNSUPPORTED, "wtq_prefill: needs head_dim 128, widths 4/4, 4/6, 6/6 or 8/8, "
                 "a power-of-two page size >= 16, at most 8 query heads per kv head and 16-byte "
                 "aligned pages");
-  if (cudaMemsetAsync(p.work_counter, 0, 256, stream) != cudaSuccess)
-    return check_cuda(cudaGetLastError(), "wtq_prefill: counter reset");
   // balanced schedule: a row's slots that no piece writes must read as empty (l = 0)
-  if (balanced && cudaMemsetAsync(p.part_l, 0, rows * splits * sizeof(float), stream) != cudaSuccess)
-    return check_cuda(cudaGetLastError(), "wtq_prefill: chunk state reset");
+  const int64_t zero_words = balanced ? (int64_t)rows * splits : 0;
   // rotation of the B * Q * Hq query rows (exp2 domain) and the lookup tables
   ScanSetup setup = {nullptr, (uint32_t *)p.lut, k_side->centroids, v_side->centroids, k_side->bw,
                      v_side->bw, mma_lut_words(k_side->bw, v_side->bw)};
   const float q_scale = scale * 1.4426950408889634f;
   if (rows_mma_rotate_eligible(q, q_strides[0], q_strides[1], Hq, D, total_rows, k_side->Pi, q_rot)) {
-    if (int rc = launch_rotate_rows_mma(q, dtype, k_side->Pi, q_scale, total_rows, q_rot, setup, status,
-                                        stream))
+    if (int rc = launch_rotate_rows_mma(q, dtype, k_side->Pi, q_scale, total_rows, q_rot, setup, p.part_l,
+                                        zero_words, p.work_counter, status, stream))
       return rc;
-  } else if (int rc = launch_rotate_q(q, dtype, q_strides, k_side->Pi, q_scale, B * Q, Hq, D, q_rot,
-                                      nullptr, chunk_tokens, max_tokens, setup, stream)) {
-    return rc;
+  } else {
+    if (cudaMemsetAsync(p.work_counter, 0, 256, stream) != cudaSuccess)
+      return check_cuda(cudaGetLastError(), "wtq_prefill: counter reset");
+    if (zero_words && cudaMemsetAsync(p.part_l, 0, zero_words * sizeof(float), stream) != cudaSuccess)
+      return check_cuda(cudaGetLastError(), "wtq_prefill: chunk state reset");
+    if (int rc = launch_rotate_q(q, dtype, q_strides, k_side->Pi, q_scale, B * Q, Hq, D, q_rot,
+                                 nullptr, chunk_tokens, max_tokens, setup, stream))
+      return rc;
   }
   int rc = WTQ_ERR_UNSUPPORTED;
   if (p.k.bw == 4 && p.v.bw == 4) rc = pf::launch<4, 4>(p, stream);

@@ -61,6 +61,11 @@ struct Params {
   uint32_t *lut;
   const float *cent_k, *cent_v;
   int bw_k, bw_v, lut_words;
+  // rotate also clears the counters and chunk sums of the kernel after it (two memsets of
+  // their own took 4-5 us of a 305 us call)
+  float *zero;
+  int64_t zero_words;
+  int32_t *counter;          // 64 words
   int32_t *status;
 };
 
@@ -113,6 +118,9 @@ __global__ void __launch_bounds__(kThreads, 1) rows_kernel(Params p) {
     if (p.lut != nullptr)
       for (int e = blockIdx.x * kThreads + tid; e < p.lut_words; e += gridDim.x * kThreads)
         p.lut[e] = mma::lut_word(e, p.bw_k, p.bw_v, p.cent_k, p.cent_v);
+    for (int64_t e = (int64_t)blockIdx.x * kThreads + tid; e < p.zero_words; e += (int64_t)gridDim.x * kThreads)
+      p.zero[e] = 0.f;
+    if (blockIdx.x == 0 && tid < 64) p.counter[tid] = 0;
   }
   // ---- the rotation, one shared-memory row per output coordinate c, contraction
   // index d along the row
@@ -352,8 +360,10 @@ bool rows_mma_rotate_eligible(const void *q, int64_t row_stride, int64_t head_st
 }
 
 int launch_rotate_rows_mma(const void *q, int dtype, const float *Pi, float mult, int64_t rows,
-                           float *q_rot, const ScanSetup &setup, int32_t *status, cudaStream_t stream) {
+                           float *q_rot, const ScanSetup &setup, float *zero, int64_t zero_words,
+                           int32_t *counter, int32_t *status, cudaStream_t stream) {
   rows::Params p = {};
+  p.zero = zero; p.zero_words = zero_words; p.counter = counter;
   p.q = q; p.in_dtype = dtype; p.mult = mult; p.Pi = Pi; p.out = q_rot; p.out_dtype = WTQ_F32;
   p.rows = rows; p.lut = setup.lut; p.cent_k = setup.cent_k; p.cent_v = setup.cent_v;
   p.bw_k = setup.bw_k; p.bw_v = setup.bw_v; p.lut_words = setup.lut_words; p.status = status;
