@@ -98,4 +98,21 @@ __device__ __forceinline__ float warp_max(float v) {
   return v;
 }
 
+// ---- two fp32 values in a 64-bit register -----------------------------------
+// Two independent fused multiply-adds, each rounded as fmaf rounds.
+__device__ __forceinline__ void fma2(uint64_t &c, uint64_t a, uint64_t b) {
+  asm("fma.rn.f32x2 %0, %1, %2, %0;\n" : "+l"(c) : "l"(a), "l"(b));
+}
+__device__ __forceinline__ uint64_t pair(float x, float y) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};\n" : "=l"(r) : "f"(x), "f"(y));
+  return r;
+}
+__device__ __forceinline__ uint64_t twice(float x) { return pair(x, x); }
+__device__ __forceinline__ float2 halves(uint64_t x) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;\n" : "=f"(r.x), "=f"(r.y) : "l"(x));
+  return r;
+}
+
 }  // namespace wtq

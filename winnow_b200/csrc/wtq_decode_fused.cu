@@ -1,12 +1,12 @@
 // Decode attention in ONE launch: for calls whose work fits about one block per
 // multiprocessor, where the split-K path (rotation, page scan, merge: three
 // dependent kernels) is bound by the kernels' own latencies, and for head_dim
-// 64, which the split-K tensor-core scan does not serve.
+// 64, which the split-K tensor-core scan does not serve (in fp32: wtq_scan32.cuh).
 //
 // A cluster of c blocks (c = 1, 2, 4, 8) owns one (sequence, kv head) group.
 // Every block rotates the group's query rows itself, each of its warps scans a
-// contiguous share of the sequence's 32-token windows exactly as the split-K
-// scan does (wtq_scan.cuh), the block merges its warps' states through shared
+// contiguous share of the sequence's 32-token windows (head_dim 128 exactly as the
+// split-K scan does, wtq_scan.cuh), the block merges its warps' states through shared
 // memory, the blocks of the cluster exchange theirs through distributed shared
 // memory, and each of them rotates 1/c of the output coordinates back and
 // stores them.  Nothing goes through global memory but the inputs and the
@@ -19,7 +19,7 @@
 #include <atomic>
 #include <mutex>
 
-#include "wtq_scan.cuh"
+#include "wtq_scan32.cuh"
 
 namespace wtq {
 namespace fused {
@@ -32,10 +32,10 @@ constexpr uint32_t kBase = 2048;            // dynamic shared memory must start 
 constexpr int kHeads = 8;                   // query heads of a group (MMA columns)
 constexpr int kRotThreads = 256;            // threads of the two rotations
 
-// Row stride of the value rows in a tile slot: padded so that the lanes' loads
-// (group g: D/8 codes, t: two rows further) fall into different banks.
+// Row stride of the value rows in a tile slot.  head_dim 128: padded so that the lanes'
+// loads (group g: D/8 codes, t: two rows further) fall into different banks.
 constexpr int vrow(int D, int bw) {
-  return D == 128 ? (bw == 4 ? 80 : bw == 6 ? 112 : 144) : (bw == 8 ? 80 : 48);
+  return D == 128 ? (bw == 4 ? 80 : bw == 6 ? 112 : 144) : 8 * bw;
 }
 
 template <int D, int BWK, int BWV> struct Cfg : Slot<D, BWK, BWV, vrow(D, BWV)> {
@@ -43,11 +43,15 @@ template <int D, int BWK, int BWV> struct Cfg : Slot<D, BWK, BWV, vrow(D, BWV)> 
   static constexpr int kPart = D * D / kRotThreads;             // coordinates per thread of the query rotation
   static constexpr int kQRow = D + 4 * (D / kPart);             // staged query row (4 words of pad per part)
   static constexpr uint32_t kQ = kBase;                         // staged queries; later the block's merged state
-  static constexpr uint32_t kQRot = kQ + kHeads * kQRow * 4;    // rotated queries [8][D]; later the sums a
-  static constexpr uint32_t kML = kQRot + kHeads * D * 4;       // the block's m[8], l[8]
+  static constexpr bool kFp32 = D == 64;                        // which scan: wtq_scan32.cuh or wtq_scan.cuh
+  static constexpr uint32_t kQRot = kQ + kHeads * kQRow * 4;    // rotated queries; later the sums a
+  static constexpr uint32_t kQRotBytes = 4 * (kFp32 ? scan32::kQueryWords : kHeads * D);
+  static constexpr uint32_t kML = kQRot + kQRotBytes;           // the block's m[8], l[8]
   static constexpr uint32_t kRings = (kML + 2 * kHeads * 4 + 127) / 128 * 128;
-  static constexpr int kRing = 2 * kTilesPerIter * Base::kSlot; // two windows per warp
-  static constexpr uint32_t kLutBytes = cmax(lut_entries(BWK), lut_entries(BWV)) * 256u;
+  static constexpr int kRingWindows = 2 * kTilesPerIter * Base::kSlot;              // two windows per warp
+  static constexpr int kRing = kRingWindows + (kFp32 ? (int)scan32::kWeights : 0);  // and the value weights
+  static constexpr uint32_t kLutBytes =
+      kFp32 ? scan32::table_bytes(BWK, BWV) : cmax(lut_entries(BWK), lut_entries(BWV)) * 256u;
   static constexpr int kRingsBelow = (int)((kLutAddr - kRings) / kRing);
   static constexpr int kRingsAbove = (int)((kSmemLimit - kLutAddr - kLutBytes) / kRing);
   static constexpr int kWarps = cmin(12, kRingsBelow + kRingsAbove);
@@ -56,7 +60,7 @@ template <int D, int BWK, int BWV> struct Cfg : Slot<D, BWK, BWV, vrow(D, BWV)> 
       kLutAddr + kLutBytes + (uint32_t)cmax(kWarps - kRingsBelow, 0) * kRing;
   // a warp's state (acc [8][D], m, l) replaces its ring after the scan; the output
   // rotation's partial sums replace the rings below the tables after the merge
-  static_assert(kRing >= kHeads * D * 4 + 2 * kHeads * 4, "state fits the ring");
+  static_assert(kRing >= kHeads * D * 4 + 2 * kHeads * 4 && kRing % 16 == 0, "state fits the ring");
   static_assert(kRings + kRotThreads * kHeads * 4 <= kLutAddr, "partial sums fit");
   static_assert(kThreads >= kRotThreads && kDynamic <= kSmemLimit, "shared memory budget");
   __device__ static uint32_t ring_address(int w) {
@@ -126,7 +130,9 @@ __global__ void __launch_bounds__(Cfg<D, BWK, BWV>::kThreads, 1) decode_fused_ke
   // a lane makes the words of 32 (index, side) pairs at a time, the warp spreads each over its 32 banks
   constexpr int kPairs = (int)(C::kLutBytes / 128);
   for (int p0 = 32 * warp; p0 < kPairs; p0 += 32 * C::kWarps) {
-    const uint32_t word = mma::lut_word((p0 + lane) * 32, BWK, BWV, p.k.centroids, p.v.centroids);
+    uint32_t word;
+    if constexpr (C::kFp32) word = scan32::table_word(p0 + lane, BWK, BWV, p.k.centroids, p.v.centroids);
+    else word = mma::lut_word((p0 + lane) * 32, BWK, BWV, p.k.centroids, p.v.centroids);
 #pragma unroll
     for (int i = 0; i < 32; ++i) sts32(lut + 128u * (p0 + i) + 4u * lane, __shfl_sync(kFull, word, i));
   }
@@ -242,59 +248,75 @@ __global__ void __launch_bounds__(Cfg<D, BWK, BWV>::kThreads, 1) decode_fused_ke
     for (int h = 0; h < kHeads; ++h) {
 #pragma unroll
       for (int o = 1; o < D / C::kPart; o <<= 1) acc[h] += __shfl_xor_sync(kFull, acc[h], o);
-      if (rpart == 0) sts_f(kqrot + 4u * (h * D + rc), acc[h] * p.q_scale);
+      if (rpart == 0)
+        sts_f(kqrot + 4u * (C::kFp32 ? scan32::query_word(rc, h) : (uint32_t)(h * D + rc)), acc[h] * p.q_scale);
     }
   }
   __syncthreads();
 
-  // ---- scan --------------------------------------------------------------------
-  ScanState<D> st;
-#pragma unroll
-  for (int ks = 0; ks < D / 16; ++ks) {                         // head g, coordinates (D/4)t + 4ks ..
-    const float4 x = lds_f4(kqrot + 4u * (g * D + (D / 4) * t + 4 * ks));
-    st.qf[ks][0] = pack_half2(x.x, x.y);
-    st.qf[ks][1] = pack_half2(x.z, x.w);
-  }
-  st.clear();
-  const float *q0 = reinterpret_cast<const float *>(dyn_smem + (kqrot - smem));
+  // ---- scan: this warp's windows; its state then replaces its ring -----------------
   const uint32_t sel_k = lut | (uint32_t)(lane << 2), sel_v = sel_k | 0x80u;
   const int n_full = tok1 > tok0 ? (tok1 - tok0) / kIterTokens : 0;
   const int n_iter = (tiles + kTilesPerIter - 1) / kTilesPerIter;
-  for (int it = 0; it < n_iter; ++it) {
-    issue_window();
-    cp_async_wait<1>();
+  auto walk = [&](auto window) {                                // window(slots, first token, refused tiles, whole)
+    for (int it = 0; it < n_iter; ++it) {
+      issue_window();
+      cp_async_wait<1>();
+      __syncwarp();
+      const int half = it & 1;
+      const uint32_t refused = (bad >> (2 * half)) & 3u;
+      window(ring + (uint32_t)(half * kTilesPerIter) * C::kSlot, tok0 + it * kIterTokens, refused,
+             it < n_full && refused == 0u);
+      __syncwarp();
+    }
+    cp_async_wait<0>();
     __syncwarp();
-    const int half = it & 1;
-    const uint32_t slot0 = ring + (uint32_t)(half * kTilesPerIter) * C::kSlot;
-    const uint32_t refused = (bad >> (2 * half)) & 3u;
-    if (it < n_full && refused == 0u)
-      scan_window<typename C::Base, false>(st, slot0, 0, 0, 3u, g, t, sel_k, sel_v, q0, p.n_rep, p.k.centroids);
-    else
-      scan_window<typename C::Base, true>(st, slot0, tok0 + it * kIterTokens, tok1, ~refused & 3u, g, t, sel_k,
-                                          sel_v, q0, p.n_rep, p.k.centroids);
-    __syncwarp();
-  }
-  cp_async_wait<0>();
-  __syncwarp();
-
-  // ---- merge of the block's warps -------------------------------------------------
+  };
+  if constexpr (C::kFp32) {
+    scan32::State st;
+    st.clear();
+    walk([&](uint32_t slots, int first, uint32_t refused, bool) {
+      scan32::window<typename C::Base>(st, slots, first, tok1, ~refused & 3u, lane, sel_k, sel_v, kqrot,
+                                       ring + C::kRingWindows);
+    });
+    scan32::store_state(st, ring, lane);
+  } else {
+    ScanState<D> st;
 #pragma unroll
-  for (int o = 4; o < 32; o <<= 1) {
-    st.l0 += __shfl_xor_sync(kFull, st.l0, o);
-    st.l1 += __shfl_xor_sync(kFull, st.l1, o);
-  }
+    for (int ks = 0; ks < D / 16; ++ks) {                       // head g, coordinates (D/4)t + 4ks ..
+      const float4 x = lds_f4(kqrot + 4u * (g * D + (D / 4) * t + 4 * ks));
+      st.qf[ks][0] = pack_half2(x.x, x.y);
+      st.qf[ks][1] = pack_half2(x.z, x.w);
+    }
+    st.clear();
+    const float *q0 = reinterpret_cast<const float *>(dyn_smem + (kqrot - smem));
+    walk([&](uint32_t slots, int first, uint32_t refused, bool whole) {
+      if (whole)
+        scan_window<typename C::Base, false>(st, slots, 0, 0, 3u, g, t, sel_k, sel_v, q0, p.n_rep, p.k.centroids);
+      else
+        scan_window<typename C::Base, true>(st, slots, first, tok1, ~refused & 3u, g, t, sel_k, sel_v, q0, p.n_rep,
+                                            p.k.centroids);
+    });
 #pragma unroll
-  for (int e = 0; e < 2; ++e) {
-    const uint32_t dst = ring + 4u * ((2 * t + e) * D + (D / 8) * g);
+    for (int o = 4; o < 32; o <<= 1) {
+      st.l0 += __shfl_xor_sync(kFull, st.l0, o);
+      st.l1 += __shfl_xor_sync(kFull, st.l1, o);
+    }
 #pragma unroll
-    for (int j = 0; j < D / 16; j += 2)
-      asm volatile("st.shared.v4.f32 [%0], {%1,%2,%3,%4};\n" ::"r"(dst + 8u * j), "f"(st.acc[j][e]),
-                   "f"(st.acc[j][2 + e]), "f"(st.acc[j + 1][e]), "f"(st.acc[j + 1][2 + e]) : "memory");
-    if (g == 0) {
-      sts_f(ring + 4u * (kHeads * D + 2 * t + e), e ? st.M1 : st.M0);
-      sts_f(ring + 4u * (kHeads * D + kHeads + 2 * t + e), e ? st.l1 : st.l0);
+    for (int e = 0; e < 2; ++e) {
+      const uint32_t dst = ring + 4u * ((2 * t + e) * D + (D / 8) * g);
+#pragma unroll
+      for (int j = 0; j < D / 16; j += 2)
+        asm volatile("st.shared.v4.f32 [%0], {%1,%2,%3,%4};\n" ::"r"(dst + 8u * j), "f"(st.acc[j][e]),
+                     "f"(st.acc[j][2 + e]), "f"(st.acc[j + 1][e]), "f"(st.acc[j + 1][2 + e]) : "memory");
+      if (g == 0) {
+        sts_f(ring + 4u * (kHeads * D + 2 * t + e), e ? st.M1 : st.M0);
+        sts_f(ring + 4u * (kHeads * D + kHeads + 2 * t + e), e ? st.l1 : st.l0);
+      }
     }
   }
+
+  // ---- merge of the block's warps -------------------------------------------------
   // this block's columns of Pi_V for the output rotation: requested now, used after the merge
   const int cols = D / c, parts = kRotThreads / cols, rows_of = D / parts;   // threads = (part, column)
   const int ocol = tid % cols, opart = tid / cols;
@@ -481,9 +503,8 @@ template <int D> int launch_widths(const Params &p, int B, int Hkv, int cluster,
 // Blocks per group of the one-launch path; 0: the split-K path serves the call
 // better.  Lengths are taken at the page table's full width.
 //
-// The cluster is the largest of 1, 2, 4, 8 with all groups resident at once
-// (16 groups of 5000 tokens, head_dim 64: 20.3 / 14.5 / 11.2 us with 1 / 2 / 4 blocks,
-// 17.6 with 8, of which only part run at a time) and whose warps have about half a window each or more: at 1024 tokens
+// The cluster is the largest of 1, 2, 4, 8 with all groups resident at once and whose warps
+// have about half a window each or more: at 1024 tokens
 // and 2 groups 14.1 / 12.3 / 11.0 / 10.9 us with 1 / 2 / 4 / 8 blocks, at 200
 // tokens and 8 groups 10.5 / 11.0 / 10.6 / 12.1; a second round of blocks costs
 // more than it brings (32 groups of 8192 tokens: 22.4 us with 4, 49 with 8), and

@@ -101,20 +101,6 @@ __device__ __forceinline__ void expand(const uint32_t *w, const float *cent, flo
     expand<BW, D, I + 1>(w, cent, y);
   }
 }
-// Two independent fused multiply-adds, each rounded as fmaf rounds.
-__device__ __forceinline__ void fma2(uint64_t &c, uint64_t a, uint64_t b) {
-  asm("fma.rn.f32x2 %0, %1, %2, %0;\n" : "+l"(c) : "l"(a), "l"(b));
-}
-__device__ __forceinline__ uint64_t twice(float x) {
-  uint64_t r;
-  asm("mov.b64 %0, {%1, %1};\n" : "=l"(r) : "f"(x));
-  return r;
-}
-__device__ __forceinline__ float2 halves(uint64_t x) {
-  float2 r;
-  asm("mov.b64 {%0, %1}, %2;\n" : "=f"(r.x), "=f"(r.y) : "l"(x));
-  return r;
-}
 
 template <int BW, int D>
 __global__ void __launch_bounds__(kThreads) dequant_tiled_kernel(DequantParams p) {

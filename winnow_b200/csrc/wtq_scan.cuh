@@ -1,9 +1,8 @@
-// The page scan of the tensor-core decode kernels, in the parts their two
-// schedules share: how a 16-token tile lies in shared memory, the fragments of
-// the score and value MMAs built from packed codes, and one 32-token window of
-// the online softmax.  Used by wtq_decode_mma.cu (split-K over all
-// multiprocessors, head_dim 128) and wtq_decode_fused.cu (one launch per call,
-// head_dim 64 and 128).
+// The page scan of the tensor-core decode kernels at head_dim 128, in the parts
+// their two schedules share: how a 16-token tile lies in shared memory, the
+// fragments of the score and value MMAs built from packed codes, and one 32-token
+// window of the online softmax.  Used by wtq_decode_mma.cu (split-K over all
+// multiprocessors) and wtq_decode_fused.cu (one launch per call).
 #pragma once
 
 #include <type_traits>
@@ -64,7 +63,7 @@ __device__ __forceinline__ void value_mmas(uint32_t rows, int g, uint32_t sel, u
                                            uint32_t pb1, float (&acc)[D / 16][4]) {
   constexpr int NB8 = D / 8 * BW / 8;               // bytes of the lane's D / 8 codes
   if constexpr (BW == 4) {
-    constexpr int NW = NB8 / 4;                     // 2 at head_dim 128, 1 at 64
+    constexpr int NW = NB8 / 4;
     const uint32_t at = rows + g * NB8;
     uint32_t wa[NW], wb[NW], wc[NW], wd[NW];
     load_words<NB8>(at, wa);
@@ -101,42 +100,25 @@ __device__ __forceinline__ void value_mmas(uint32_t rows, int g, uint32_t sel, u
       for (int j = 0; j < 4; ++j) mma16816(acc[4 * h + j], f[j][0], f[j][1], f[j][2], f[j][3], pb0, pb1);
     }
   } else {
-    constexpr int NW = (NB8 + 3) / 4;
+    constexpr int NW = NB8 / 4;
     uint32_t wa[NW], wb[NW], wc[NW], wd[NW];
-    if constexpr (NB8 % 4 == 0) {
-      const uint32_t at = rows + g * NB8;
-      load_words<NB8>(at, wa);
-      load_words<NB8>(at + VROW, wb);
-      load_words<NB8>(at + 8 * VROW, wc);
-      load_words<NB8>(at + 9 * VROW, wd);
-    } else {                                        // 6 bytes (6-bit, head_dim 64): half-word aligned
-      static_assert(NB8 == 6, "six bytes");
-      const uint32_t at = rows + ((g * NB8) & ~3u), sh = (g & 1) * 16;
-      auto six = [&](uint32_t a, uint32_t (&w)[NW]) {
-        const uint32_t x = lds32(a), y = lds32(a + 4);
-        w[0] = __funnelshift_r(x, y, sh);
-        w[1] = y >> sh;
-      };
-      six(at, wa);
-      six(at + VROW, wb);
-      six(at + 8 * VROW, wc);
-      six(at + 9 * VROW, wd);
-    }
+    const uint32_t at = rows + g * NB8;
+    load_words<NB8>(at, wa);
+    load_words<NB8>(at + VROW, wb);
+    load_words<NB8>(at + 8 * VROW, wc);
+    load_words<NB8>(at + 9 * VROW, wd);
     auto one = [&](auto jc) {
       constexpr int j = decltype(jc)::value;
-      if constexpr (j < D / 16)
-        mma16816(acc[j],
-                 join(lut_code<BW, 2 * j>(wa, sel), lut_code<BW, 2 * j>(wb, sel)),
-                 join(lut_code<BW, 2 * j + 1>(wa, sel), lut_code<BW, 2 * j + 1>(wb, sel)),
-                 join(lut_code<BW, 2 * j>(wc, sel), lut_code<BW, 2 * j>(wd, sel)),
-                 join(lut_code<BW, 2 * j + 1>(wc, sel), lut_code<BW, 2 * j + 1>(wd, sel)), pb0, pb1);
+      mma16816(acc[j],
+               join(lut_code<BW, 2 * j>(wa, sel), lut_code<BW, 2 * j>(wb, sel)),
+               join(lut_code<BW, 2 * j + 1>(wa, sel), lut_code<BW, 2 * j + 1>(wb, sel)),
+               join(lut_code<BW, 2 * j>(wc, sel), lut_code<BW, 2 * j>(wd, sel)),
+               join(lut_code<BW, 2 * j + 1>(wc, sel), lut_code<BW, 2 * j + 1>(wd, sel)), pb0, pb1);
     };
     one(std::integral_constant<int, 0>{}); one(std::integral_constant<int, 1>{});
     one(std::integral_constant<int, 2>{}); one(std::integral_constant<int, 3>{});
-    if constexpr (D > 64) {
-      one(std::integral_constant<int, 4>{}); one(std::integral_constant<int, 5>{});
-      one(std::integral_constant<int, 6>{}); one(std::integral_constant<int, 7>{});
-    }
+    one(std::integral_constant<int, 4>{}); one(std::integral_constant<int, 5>{});
+    one(std::integral_constant<int, 6>{}); one(std::integral_constant<int, 7>{});
   }
 }
 
@@ -179,10 +161,8 @@ __device__ __forceinline__ void key_mmas(uint32_t at, uint32_t sel, const uint32
     };
     one(std::integral_constant<int, 0>{}); one(std::integral_constant<int, 1>{});
     one(std::integral_constant<int, 2>{}); one(std::integral_constant<int, 3>{});
-    if constexpr (D > 64) {
-      one(std::integral_constant<int, 4>{}); one(std::integral_constant<int, 5>{});
-      one(std::integral_constant<int, 6>{}); one(std::integral_constant<int, 7>{});
-    }
+    one(std::integral_constant<int, 4>{}); one(std::integral_constant<int, 5>{});
+    one(std::integral_constant<int, 6>{}); one(std::integral_constant<int, 7>{});
   }
 #pragma unroll
   for (int e = 0; e < 4; ++e) {
