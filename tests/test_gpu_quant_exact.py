@@ -6,7 +6,7 @@ import pytest
 import torch
 
 from oracle import tq_oracle as orc
-from winnow_b200.cache import _get_quantizer
+from winnow_b200.cache import TurboQuantMSE, _get_quantizer
 from winnow_b200.packed_backend import append_tokens
 from winnow_b200.packing import unpack
 
@@ -40,10 +40,7 @@ def test_widths_and_special_rows(bw):
     check(x, bw)
 
 
-@pytest.mark.parametrize("bw", [4, 8])
-def test_coordinates_on_boundaries(bw):
-    """x = y Pi with y on (or a few fp32 steps beside) boundaries: the rotation
-    returns to within an ulp or so of them, on either side."""
+def on_boundaries(bw):
     oq = orc.OracleQuantizer.get(bw, 128, 42)
     g = torch.Generator().manual_seed(99)
     edges = oq.boundaries
@@ -54,7 +51,27 @@ def test_coordinates_on_boundaries(bw):
     y[:, :24] = edges.double()[pick] * (1 + torch.randint(-3, 4, (4096, 24), generator=g) * 2.0 ** -24)
     rest = (1.0 - (y[:, :24] ** 2).sum(1, keepdim=True)).clamp_min(1e-3).sqrt()
     y[:, 24:] *= rest / y[:, 24:].norm(dim=1, keepdim=True)          # |y| = 1: division leaves it in place
-    check((y @ oq.Pi.double()).float(), bw)
+    return (y @ oq.Pi.double()).float()
+
+
+@pytest.mark.parametrize("bw", [4, 8])
+def test_coordinates_on_boundaries(bw):
+    """x = y Pi with y on (or a few fp32 steps beside) boundaries: the rotation
+    returns to within an ulp or so of them, on either side."""
+    check(on_boundaries(bw), bw)
+
+
+@pytest.mark.parametrize("longer", [0.0625, 3.0, 256.0, 4096.0])
+@pytest.mark.parametrize("bw", [4, 8])
+def test_matrix_with_rows_of_any_length(bw, longer):
+    """Not a rotation: coordinates, boundaries and rounding errors all grow with the rows
+    (4096: operands beyond fp16)."""
+    x, oq, tq = on_boundaries(bw), orc.OracleQuantizer(bw, 128, 42), TurboQuantMSE(bw, 128, DEV)
+    for t in (oq, tq):
+        t.Pi, t.boundaries = (t.Pi * longer).contiguous(), (t.boundaries * longer).contiguous()
+    idx, norm = tq.quantize(x.to(DEV))
+    ref_idx, ref_norm = oq.quantize(x)
+    assert torch.equal(idx.cpu(), ref_idx) and torch.equal(norm.cpu(), ref_norm)
 
 
 def test_odd_strides_and_unaligned_destinations():

@@ -24,7 +24,8 @@
 // third used): dependent divisions, MMA chains, one round of FMA chains; a form with
 // block-wide phases and barriers took 130 us (268).
 //
-// kMargin: with sum_d |x_d| |Pi_cd| <= |x| |Pi_c| = 1, the chain is within
+// kMargin is for rows of Pi no longer than 1, as a rotation's are; longer ones (any matrix
+// is accepted) scale it, since every term below grows with |Pi_c|.  With sum_d |x_d| |Pi_cd| <= |x| |Pi_c| = 1, the chain is within
 // 128 * 2^-24 = 7.6e-6 of the exact sum; the split operands leave out 3 * 2^-22
 // = 7e-7; each of the 8 accumulating high x high MMAs adds 17 terms aligned to the
 // largest (below 1) and cut at 24 bits, at most 17 * 2^-24 = 1.0e-6 each, and the
@@ -60,6 +61,7 @@ struct Smem {
   float2 around[256];                                 // boundaries below and above bucket k (-inf, +inf at the ends)
   uint8_t cell[kCells];                               // bucket of the lower end of each cell
   int crowded;                                        // a cell holds more than one boundary: search instead
+  int longest;                                        // the largest |Pi_c|^2, as bits
   WarpSmem warp[kWarps];
 };
 
@@ -155,6 +157,7 @@ __global__ void __launch_bounds__(kThreads, 1) quant_mma_kernel(QuantJob job) {
   WarpSmem &w = s.warp[warp];
   // ---- constants: Pi as B fragments (n = output coordinate, k = input coordinate),
   // boundaries, cells ------------------------------------------------------------------
+  float *squares = reinterpret_cast<float *>(s.warp);  // of each fragment, until the warps' tiles are used
 #pragma unroll 4
   for (int e = warp; e < 128; e += kWarps) {
     const int nt = e >> 3, ks = e & 7;
@@ -164,11 +167,23 @@ __global__ void __launch_bounds__(kThreads, 1) quant_mma_kernel(QuantJob job) {
     split2(p.x * kScale, p.y * kScale, f.x, f.z);
     split2(q.x * kScale, q.y * kScale, f.y, f.w);
     s.pi[nt][ks][lane] = f;
+    squares[e * 32 + lane] = fmaf(p.x, p.x, fmaf(p.y, p.y, fmaf(q.x, q.x, q.y * q.y)));
   }
   for (int e = tid; e <= nbounds; e += kThreads)
     s.around[e] = make_float2(e > 0 ? __ldg(a.q.bounds + e - 1) : -INFINITY, e < nbounds ? __ldg(a.q.bounds + e) : INFINITY);
-  if (tid == 0) s.crowded = 0;
+  if (tid == 0) s.crowded = s.longest = 0;
   __syncthreads();
+  if (tid >= kThreads - 128) {                        // (the threads with fewest cells)
+    const int c = tid - (kThreads - 128);
+    float sum = 0.f;
+#pragma unroll
+    for (int ks = 0; ks < 8; ++ks) {
+      const float4 v = *reinterpret_cast<const float4 *>(squares + ((c >> 3) * 8 + ks) * 32 + (c & 7) * 4);
+      sum += (v.x + v.y) + (v.z + v.w);
+    }
+    const int most = __reduce_max_sync(kFull, __float_as_int(fabsf(sum)));       // (a NaN beats every number)
+    if (lane == 0) atomicMax(&s.longest, most);
+  }
   // (cells start at multiples of 2^-10, exact in fp32)
   for (int e = tid; e < kCells; e += kThreads)
     s.cell[e] = (uint8_t)(e == 0 ? 0 : bucket(s, nbounds, (float)e * (1.f / kCells) - 0.5f));
@@ -177,6 +192,8 @@ __global__ void __launch_bounds__(kThreads, 1) quant_mma_kernel(QuantJob job) {
     if ((e == kCells - 1 ? nbounds : s.cell[e + 1]) - s.cell[e] > 1) s.crowded = 1;
   __syncthreads();
   const bool crowded = s.crowded != 0;
+  const float longest = __int_as_float(s.longest);
+  const float margin = longest <= 1.0001f ? kMargin : kMargin * sqrtf(longest);   // (NaN stays: every chain runs)
   asm volatile("griddepcontrol.wait;\n" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
 
@@ -288,7 +305,7 @@ __global__ void __launch_bounds__(kThreads, 1) quant_mma_kernel(QuantJob job) {
           k[e] = bucket(s, nbounds, y);
           edge = s.around[k[e]];
         }
-        doubt[e] = !(y - edge.x > kMargin) || !(edge.y - y > kMargin);
+        doubt[e] = !(y - edge.x > margin) || !(edge.y - y > margin);
       }
 #pragma unroll
       for (int e = 0; e < 8; e += 2)                             // rows g, g + 8; coordinates 2t, 2t + 1
