@@ -1,5 +1,6 @@
-"""head_dim 64 decodes in fp32 whatever the size of the values: queries, centroids,
-probabilities and value weights are 32-bit floats, against 64-bit arithmetic."""
+"""Calls that decode in fp32 throughout (queries, centroids, probabilities and value
+weights are 32-bit floats), against 64-bit arithmetic: head_dim 64 whatever the size of the
+values, head_dim 128 with layouts the tensor-core scan does not take."""
 import math
 
 import pytest
@@ -8,7 +9,7 @@ import torch
 import cases
 from helpers import oracle_case, to_device
 from oracle import tq_oracle as orc
-from winnow_b200.packed_attention_cuda import packed_decode_attention
+from winnow_b200.packed_attention_cuda import decode_workspace, packed_decode_attention
 from winnow_b200.packing import unpack
 
 pytestmark = pytest.mark.gpu
@@ -50,11 +51,35 @@ def test_fp32_against_64_bits(widths, heads, v_scale, q_scale):
     ref, size, top = exact(q.cuda(), kv, scale)
     got = packed_decode_attention(q.cuda(), kv, scale)
     assert got.dtype == torch.float32
-    # u = 2^-24.  A score sums 64 products twice (rotation, then centroids) and takes three more
-    # roundings: off by at most 131 u |q| |k|; a probability by that times ln 2 and by 2^-22 for
-    # exp2, its quotient by twice as much.  The value sum of 3001 keys takes a rounding per key of
-    # a warp's share (at most 251), some 20 to merge and 64 to rotate back.
+    check(got, ref, size, top, 64, 251)
+
+
+def check(got, ref, size, top, D, keys):
+    # u = 2^-24.  A score sums D products twice (rotation, then centroids) and takes three more
+    # roundings: off by at most (2 D + 3) u |q| |k|; a probability by that times ln 2 and by 2^-22
+    # for exp2, its quotient by twice as much.  The value sum takes a rounding per key of a chain
+    # (`keys`: a warp's share of 3001, or all), some 20 to merge and D to rotate back.
     u = 2.0 ** -24
-    bound = 2 * (131 * u * math.log(2) * top + 2.0 ** -22) + (251 + 20 + 64) * u
+    bound = 2 * ((2 * D + 3) * u * math.log(2) * top + 2.0 ** -22) + (keys + 20 + D) * u
     err = (got[:, :, 0].double() - ref).norm(dim=-1)
     assert (err <= bound * size).all(), float((err / size.clamp_min(1e-300)).max() / bound)
+
+
+def test_layouts_the_tensor_core_scan_does_not_take():
+    """Pages 2^31 bytes apart, and a workspace off its alignment."""
+    c = C("far", 43, 2, 8, 2, 128, (1, 40), 16, 4, 4, 0.02)
+    q, okv, _ = oracle_case(c)
+    kv, scale = to_device(okv, "cuda"), orc.default_scale(128)
+    ref, size, top = exact(q.cuda(), kv, scale)
+    for splits in (None, 2):
+        ws = decode_workspace(2, 8, 2, 128, kv.page_table.shape[1], 16, splits or 0, "cuda")
+        off = torch.zeros(ws.numel() + 16, dtype=torch.uint8, device="cuda")[4:]
+        got = packed_decode_attention(q.cuda(), kv, scale, num_splits=splits, workspace=off)
+        check(got, ref, size, top, 128, 40)
+    P, H, S, NB = kv.k_pages.shape
+    far = torch.zeros((P - 1 << 31) + H * S * NB, dtype=torch.uint8, device="cuda")
+    far = far.as_strided((P, H, S, NB), (1 << 31, S * NB, NB, 1))
+    far.copy_(kv.k_pages)
+    kv.k_pages = far
+    for splits in (None, 2):
+        check(packed_decode_attention(q.cuda(), kv, scale, num_splits=splits), ref, size, top, 128, 40)

@@ -194,7 +194,8 @@ static int decode_common(const void *q, int dtype, const int64_t q_strides[2], v
   if (workspace_bytes < need)
     return fail(WTQ_ERR_WORKSPACE, "wtq_decode: workspace %zu < %zu bytes", workspace_bytes, need);
 
-  if (!exchange && num_splits <= 0)
+  // (a workspace off 16-byte boundaries keeps head_dim 128 on the fp32 kernels, see mma_eligible)
+  if (!exchange && num_splits <= 0 && (D == 64 || ((uintptr_t)workspace & 15) == 0))
     if (const int cluster = one_launch_cluster(p))
       return one_launch(p, cluster, q, dtype, q_strides, scale, out, out_strides, stream);
 

@@ -537,7 +537,11 @@ bool fused_eligible(const DecodeParams &p) {
          aligned(p.k.pages) && aligned(p.v.pages) && aligned(p.k.norms) && aligned(p.v.norms) &&
          aligned(p.k.Pi) && p.k.page_stride % 16 == 0 && p.k.head_stride % 16 == 0 &&
          p.v.page_stride % 16 == 0 && p.v.head_stride % 16 == 0 && p.k.norm_page_stride % 8 == 0 &&
-         p.k.norm_head_stride % 8 == 0 && p.v.norm_page_stride % 8 == 0 && p.v.norm_head_stride % 8 == 0;
+         p.k.norm_head_stride % 8 == 0 && p.v.norm_page_stride % 8 == 0 && p.v.norm_head_stride % 8 == 0 &&
+         // head_dim 128 rounds operands to 16 bits: only calls whose split-K scan does so too
+         // (mma_eligible), none that the fp32 kernels serve
+         (p.D == 64 || (p.k.page_stride < (int64_t)1 << 31 && p.v.page_stride < (int64_t)1 << 31 &&
+                        p.k.norm_page_stride < (int64_t)1 << 30 && p.v.norm_page_stride < (int64_t)1 << 30));
 }
 
 int launch_decode_fused(const DecodeParams &p, const void *q, int dtype, const int64_t q_strides[2],
