@@ -1,0 +1,51 @@
+"""What the append and the contiguous cache refuse before anything is launched, on tensors
+without storage: a kernel given these arguments would read outside its buffers."""
+from types import SimpleNamespace
+
+import pytest
+import torch
+from torch._subclasses.fake_tensor import FakeTensorMode
+
+from winnow_b200 import packed_backend as pb
+from winnow_b200.cache import TQPackedLayer
+
+
+@pytest.fixture
+def fake():
+    with FakeTensorMode():
+        yield
+
+
+def _append_args(B=4, rows=4, lens=4, device="cuda", Pi_device="cuda"):
+    D, H, n, S, P = 128, 2, 8, 16, 5
+    x = [torch.empty(B, H, n, D, dtype=torch.float16, device=device) for _ in range(2)]
+    pages = [torch.empty(P, H, S, 64, dtype=torch.uint8, device=device) for _ in range(2)]
+    norms = [torch.empty(P, H, S, dtype=torch.float16, device=device) for _ in range(2)]
+    tq = SimpleNamespace(Pi=torch.empty(D, D, device=Pi_device), centroids=torch.empty(16, device=Pi_device),
+                         boundaries=torch.empty(15, device=Pi_device), bit_width=4)
+    return [*x, pages[0], norms[0], pages[1], norms[1], torch.empty(rows, 1, dtype=torch.int32, device=device),
+            torch.empty(lens, dtype=torch.int32, device=device), tq, tq]
+
+
+@pytest.mark.parametrize("rows,lens", [(3, 4), (4, 3), (1, 1)])
+def test_append_needs_a_table_row_and_a_length_per_sequence(fake, rows, lens):
+    with pytest.raises(ValueError, match="row for each of 4"):
+        pb.AppendPlan(*_append_args(rows=rows, lens=lens))
+
+
+@pytest.mark.parametrize("k_shape,v_shape", [((3, 2, 8, 128), None), ((1, 2, 8, 128), None), ((8, 2, 8, 128), None),
+                                             ((4, 1, 8, 128), None), ((4, 2, 8, 128), (4, 2, 1, 128)),
+                                             ((4, 2, 8, 128), (1, 2, 8, 128))])
+def test_contiguous_cache_appends_only_its_own_shape(fake, monkeypatch, k_shape, v_shape):
+    """Other shapes go part by part, where assignment broadcasts them or raises."""
+    called = []
+    monkeypatch.setattr(pb, "append_tokens", lambda *a, **k: called.append(1))
+    layer = TQPackedLayer.__new__(TQPackedLayer)
+    layer._out_dim, layer._shape, layer._tq = 0, (4, 2, 128), None
+    layer._ring_len = torch.zeros(4, dtype=torch.int32, device="cuda")
+    layer._ring_table = layer._k = layer._v = (None, None)
+    ks = torch.empty(k_shape, dtype=torch.float16, device="cuda")
+    vs = torch.empty(v_shape or k_shape, dtype=torch.float16, device="cuda")
+    assert not layer._store_both(ks, vs, 0, 8) and not called
+    own = torch.empty(4, 2, 8, 128, dtype=torch.float16, device="cuda")
+    assert layer._store_both(own, own, 0, 8) and called

@@ -278,9 +278,12 @@ class TQPackedLayer(_LayerBase):
     def _store_both(self, ks, vs, pos, n) -> bool:
         """K and V of n new tokens into the rings with one fused append (the rings are
         pages of `max_cache_len` tokens, one per sequence); False where outlier
-        channels or the source type need the part-by-part form."""
+        channels, the source type or a shape other than the rings' need the part-by-part form
+        (which broadcasts, or says what does not fit)."""
+        B, H, D = self._shape
         if self._out_dim or ks.dtype != vs.dtype or ks.dtype not in (torch.float32, torch.float16,
-                                                                     torch.bfloat16):
+                                                                     torch.bfloat16) \
+                or ks.shape != (B, H, n, D) or vs.shape != ks.shape:
             return False
         from .packed_backend import append_tokens
         self._ring_len.fill_(pos + n)

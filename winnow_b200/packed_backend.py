@@ -220,6 +220,8 @@ class AppendPlan:
         if page_table.dtype != torch.int32 or seq_lens.dtype != torch.int32 \
                 or page_table.stride(-1) != 1 or not seq_lens.is_contiguous():
             raise ValueError("page_table and seq_lens must be contiguous int32")
+        if page_table.dim() != 2 or page_table.shape[0] < B or seq_lens.numel() < B:
+            raise ValueError(f"page_table and seq_lens need a row for each of {B} sequences")
         self.device = dev
         self._sides = [
             _lib.Side(pages.data_ptr(), norms.data_ptr(), pages.stride(0), pages.stride(1),
