@@ -4,6 +4,7 @@ import pytest
 import torch
 
 from oracle import tq_oracle as orc
+from winnow_b200 import _lib
 from winnow_b200.cache import TQPackedLayer
 
 pytestmark = pytest.mark.gpu
@@ -41,3 +42,9 @@ def test_shapes_that_do_not_fit_raise(shape):
         layer.update(x, x)
     assert layer.get_seq_length() == 9
     assert all(torch.equal(a, b[:, :, :9]) for a, b in zip(before, layer._k[:2] + layer._v[:2]))
+
+
+def test_quantizer_on_another_device_raises():
+    x = torch.zeros(2, 2, 3, 128, dtype=torch.float16, device=DEV)
+    with pytest.raises(_lib.BackendError):
+        TQPackedLayer(128, 4, "cpu", 32).update(x, x)

@@ -6,7 +6,7 @@ import pytest
 import torch
 from torch._subclasses.fake_tensor import FakeTensorMode
 
-from winnow_b200 import packed_backend as pb
+from winnow_b200 import _lib, packed_backend as pb
 from winnow_b200.cache import TQPackedLayer
 
 
@@ -31,6 +31,11 @@ def _append_args(B=4, rows=4, lens=4, device="cuda", Pi_device="cuda"):
 def test_append_needs_a_table_row_and_a_length_per_sequence(fake, rows, lens):
     with pytest.raises(ValueError, match="row for each of 4"):
         pb.AppendPlan(*_append_args(rows=rows, lens=lens))
+
+
+def test_append_needs_its_quantizers_on_the_device(fake):
+    with pytest.raises(_lib.BackendError):
+        pb.AppendPlan(*_append_args(Pi_device="cpu"))
 
 
 @pytest.mark.parametrize("k_shape,v_shape", [((3, 2, 8, 128), None), ((1, 2, 8, 128), None), ((8, 2, 8, 128), None),
