@@ -54,3 +54,39 @@ def test_contiguous_cache_appends_only_its_own_shape(fake, monkeypatch, k_shape,
     assert not layer._store_both(ks, vs, 0, 8) and not called
     own = torch.empty(4, 2, 8, 128, dtype=torch.float16, device="cuda")
     assert layer._store_both(own, own, 0, 8) and called
+
+
+_NO_STORAGE = """
+import sys
+sys.path[:0] = {path!r}
+import torch
+from torch._subclasses.fake_tensor import FakeTensorMode
+from test_refusals import _append_args
+from winnow_b200 import _lib, packed_attention as pa, packed_backend as pb
+host = _lib.host()
+with FakeTensorMode():
+    args = _append_args()
+    k, v, kp, kn, vp, vn, table, lens, tq, _ = args
+    q = torch.empty(4, 8, 1, 128, dtype=torch.float16, device="cuda")
+    quant = pa.Quantizer.from_tq(tq)
+    kv = pa.PackedKV(kp, kn, vp, vn, table, lens, quant, quant, 128)
+    status = torch.empty(1, dtype=torch.int32, device="cuda")
+    for call in (lambda: pb.append_tokens(*args), lambda: host.append(*args, -1, status),
+                 lambda: host.stage(k, k, v, v, q, q), lambda: host.decode(q, kv, 1.0, 0, None, None, status),
+                 lambda: host.decode(q, kv, 1.0, 4, torch.empty_like(q), None, None),
+                 lambda: host.attend(q, kv, 1.0, None)):
+        try:
+            call()
+        except Exception as e:
+            print("raised", type(e).__name__)
+"""
+
+
+def test_tensors_without_storage_raise():
+    """In a process of its own: a C++ exception that leaves the interpreter's C function ends it."""
+    import subprocess
+    import sys
+    code = _NO_STORAGE.format(path=[p for p in sys.path if p])
+    done = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=300)
+    assert done.returncode == 0, done.stderr[-2000:]
+    assert done.stdout.count("raised ") == 6, done.stdout

@@ -5,7 +5,11 @@
 //
 // Every function here is the fast path of one Python function and only ever
 // answers "done" or "not mine" (None): whatever it does not serve, malformed
-// arguments among it, goes through the Python path, which raises the errors.
+// arguments among it, goes through the Python path, which raises the errors.  C++
+// exceptions (no memory, a tensor without storage, a device that cannot be set) leave as
+// the Python exceptions that torch's own functions raise for them, and every tensor whose
+// address goes to the library is held until the call returns.
+#include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 #include <ATen/ATen.h>
 #include <ATen/cuda/CUDAContext.h>
@@ -87,9 +91,14 @@ bool side_pages(const at::Tensor &pages, const at::Tensor &norms, int64_t bw, in
 }
 
 // The rotation and one table of a quantizer (`table`: centroids or boundaries).
-bool quant_table(PyObject *quant, PyObject *table, int64_t D, int64_t extra, const at::Device &dev, int64_t &bw,
-                 const float *&Pi, const float *&values) {
+struct Quant {
+  int64_t bw = 0;
   at::Tensor pi, tab;
+};
+bool quant_table(PyObject *quant, PyObject *table, int64_t D, int64_t extra, const at::Device &dev, Quant &held,
+                 const float *&Pi, const float *&values) {
+  int64_t &bw = held.bw;
+  at::Tensor &pi = held.pi, &tab = held.tab;
   if (!int_attr(quant, N.bit_width, bw) || bw < 1 || bw > 8 || !tensor_attr(quant, N.Pi, pi) ||
       !tensor_attr(quant, table, tab))
     return false;
@@ -113,12 +122,13 @@ bool table_and_lengths(const at::Tensor &table, const at::Tensor &lens, int64_t 
 // One layer's paged packed K/V (a PackedKV) for queries of head_dim D on `dev`.
 struct Layer {
   wtq_side_t k, v;
-  at::Tensor table, lens;
+  at::Tensor kp, kn, vp, vn, table, lens;
+  Quant k_quant, v_quant;
   int64_t P, Hkv, S;
 };
 bool read_layer(PyObject *kv, int64_t B, int64_t D, const at::Device &dev, Layer &l) {
-  int64_t head_dim = 0, bw_k = 0, bw_v = 0;
-  at::Tensor kp, kn, vp, vn;
+  int64_t head_dim = 0;
+  at::Tensor &kp = l.kp, &kn = l.kn, &vp = l.vp, &vn = l.vn;
   if (!int_attr(kv, N.head_dim, head_dim) || head_dim != D || D < 1 || D > 256) return false;
   if (!tensor_attr(kv, N.k_pages, kp) || !tensor_attr(kv, N.k_norms, kn) || !tensor_attr(kv, N.v_pages, vp) ||
       !tensor_attr(kv, N.v_norms, vn) || !tensor_attr(kv, N.page_table, l.table) || !tensor_attr(kv, N.seq_lens, l.lens))
@@ -128,10 +138,10 @@ bool read_layer(PyObject *kv, int64_t B, int64_t D, const at::Device &dev, Layer
     return false;
   Ref kq(PyObject_GetAttr(kv, N.k_quant)), vq(PyObject_GetAttr(kv, N.v_quant));
   l.k.bounds = l.v.bounds = nullptr;
-  if (!kq || !vq || !quant_table(kq.o, N.centroids, D, 0, dev, bw_k, l.k.Pi, l.k.centroids) ||
-      !quant_table(vq.o, N.centroids, D, 0, dev, bw_v, l.v.Pi, l.v.centroids))
+  if (!kq || !vq || !quant_table(kq.o, N.centroids, D, 0, dev, l.k_quant, l.k.Pi, l.k.centroids) ||
+      !quant_table(vq.o, N.centroids, D, 0, dev, l.v_quant, l.v.Pi, l.v.centroids))
     return false;
-  if (!side_pages(kp, kn, bw_k, D, l.k) || !side_pages(vp, vn, bw_v, D, l.v)) return false;
+  if (!side_pages(kp, kn, l.k_quant.bw, D, l.k) || !side_pages(vp, vn, l.v_quant.bw, D, l.v)) return false;
   for (int i = 0; i < 3; ++i)
     if (kp.size(i) != vp.size(i)) return false;
   l.P = kp.size(0);
@@ -140,10 +150,9 @@ bool read_layer(PyObject *kv, int64_t B, int64_t D, const at::Device &dev, Layer
   return l.P >= 1 && l.Hkv >= 1 && l.S >= 1 && l.table.size(1) >= 1;
 }
 
-bool optional_status(PyObject *o, const at::Device &dev, int32_t *&p) {
+bool optional_status(PyObject *o, const at::Device &dev, at::Tensor &t, int32_t *&p) {
   p = nullptr;
   if (o == Py_None) return true;
-  at::Tensor t;
   if (!tensor(o, t) || t.scalar_type() != at::kInt || t.numel() < 1 || t.device() != dev) return false;
   p = t.mutable_data_ptr<int32_t>();
   return true;
@@ -158,14 +167,15 @@ PyObject *library_error(int rc) {
 // tensor, (B, Hq, 1, D) or, with `token_major`, (B, 1, Hq, D).
 PyObject *run_decode(PyObject *q_arg, PyObject *kv, PyObject *scale_arg, long splits, PyObject *out_arg, PyObject *ws_arg,
                      PyObject *status_arg, bool token_major) {
-  at::Tensor q, out, ws;
+  at::Tensor q, out, ws, status_tensor;
   if (!tensor(q_arg, q) || !q.is_cuda() || q.dim() != 4 || q.size(2) != 1 || q.stride(3) != 1) Py_RETURN_NONE;
   const int dtype = dtype_code(q.scalar_type());
   const int64_t B = q.size(0), Hq = q.size(1), D = q.size(3);
   const at::Device dev = q.device();
   Layer l;
   int32_t *status;
-  if (dtype < 0 || B < 1 || Hq < 1 || !read_layer(kv, B, D, dev, l) || Hq % l.Hkv || !optional_status(status_arg, dev, status))
+  if (dtype < 0 || B < 1 || Hq < 1 || !read_layer(kv, B, D, dev, l) || Hq % l.Hkv ||
+      !optional_status(status_arg, dev, status_tensor, status))
     Py_RETURN_NONE;
   const double scale = PyFloat_AsDouble(scale_arg);
   if (PyErr_Occurred()) {
@@ -178,51 +188,47 @@ PyObject *run_decode(PyObject *q_arg, PyObject *kv, PyObject *scale_arg, long sp
       Py_RETURN_NONE;
   }
   if (ws_arg != Py_None && (!tensor(ws_arg, ws) || ws.device() != dev)) Py_RETURN_NONE;
-  try {
-    const c10::cuda::OptionalCUDAGuard guard(dev);
-    int64_t os[2] = {Hq * D, D};
-    if (out.defined()) {
-      os[0] = out.stride(0);
-      os[1] = out.stride(1);
-    } else {
-      out = token_major ? at::empty({B, 1, Hq, D}, q.options()) : at::empty({B, Hq, 1, D}, q.options());
-    }
-    void *stream = (void *)at::cuda::getCurrentCUDAStream(dev.index()).stream();
-    const int64_t qs[2] = {q.stride(0), q.stride(1)};
-    const int W = (int)l.table.size(1), S = (int)l.S, H = (int)l.Hkv;
-    int rc = WTQ_ERR_UNSUPPORTED;
-    if (splits <= 0 && !ws.defined()) {
-      const Unlocked u;
-      rc = wtq_decode_direct(q.const_data_ptr(), dtype, qs, out.mutable_data_ptr(), os, &l.k, &l.v,
-                             l.table.const_data_ptr<int32_t>(), l.table.stride(0), l.lens.const_data_ptr<int32_t>(),
-                             (float)scale, (int)B, (int)Hq, H, (int)D, S, (int)l.P, W, status, stream);
-    }
-    if (rc == WTQ_ERR_UNSUPPORTED) {
-      if (!ws.defined()) {
-        ws = at::empty({(int64_t)wtq_decode_workspace_bytes((int)B, (int)Hq, H, (int)D, W, S, (int)splits)},
-                       q.options().dtype(at::kByte));
-        ws.narrow(0, 0, (int64_t)wtq_decode_counter_bytes((int)B, H)).zero_();
-      }
-      const Unlocked u;
-      rc = wtq_decode(q.const_data_ptr(), dtype, qs, out.mutable_data_ptr(), os, &l.k, &l.v,
-                      l.table.const_data_ptr<int32_t>(), l.table.stride(0), l.lens.const_data_ptr<int32_t>(),
-                      (float)scale, (int)B, (int)Hq, H, (int)D, S, (int)l.P, W, (int)splits, ws.mutable_data_ptr(),
-                      (size_t)ws.numel(), status, stream);
-    }
-    if (rc) return library_error(rc);
-    if (out_arg != Py_None) {
-      Py_INCREF(out_arg);
-      return out_arg;
-    }
-    return THPVariable_Wrap(std::move(out));
-  } catch (const std::exception &e) {
-    PyErr_SetString(PyExc_RuntimeError, e.what());
-    return nullptr;
+  const c10::cuda::OptionalCUDAGuard guard(dev);
+  int64_t os[2] = {Hq * D, D};
+  if (out.defined()) {
+    os[0] = out.stride(0);
+    os[1] = out.stride(1);
+  } else {
+    out = token_major ? at::empty({B, 1, Hq, D}, q.options()) : at::empty({B, Hq, 1, D}, q.options());
   }
+  void *stream = (void *)at::cuda::getCurrentCUDAStream(dev.index()).stream();
+  const int64_t qs[2] = {q.stride(0), q.stride(1)};
+  const int W = (int)l.table.size(1), S = (int)l.S, H = (int)l.Hkv;
+  int rc = WTQ_ERR_UNSUPPORTED;
+  if (splits <= 0 && !ws.defined()) {
+    const Unlocked u;
+    rc = wtq_decode_direct(q.const_data_ptr(), dtype, qs, out.mutable_data_ptr(), os, &l.k, &l.v,
+                           l.table.const_data_ptr<int32_t>(), l.table.stride(0), l.lens.const_data_ptr<int32_t>(),
+                           (float)scale, (int)B, (int)Hq, H, (int)D, S, (int)l.P, W, status, stream);
+  }
+  if (rc == WTQ_ERR_UNSUPPORTED) {
+    if (!ws.defined()) {
+      ws = at::empty({(int64_t)wtq_decode_workspace_bytes((int)B, (int)Hq, H, (int)D, W, S, (int)splits)},
+                     q.options().dtype(at::kByte));
+      ws.narrow(0, 0, (int64_t)wtq_decode_counter_bytes((int)B, H)).zero_();
+    }
+    const Unlocked u;
+    rc = wtq_decode(q.const_data_ptr(), dtype, qs, out.mutable_data_ptr(), os, &l.k, &l.v,
+                    l.table.const_data_ptr<int32_t>(), l.table.stride(0), l.lens.const_data_ptr<int32_t>(),
+                    (float)scale, (int)B, (int)Hq, H, (int)D, S, (int)l.P, W, (int)splits, ws.mutable_data_ptr(),
+                    (size_t)ws.numel(), status, stream);
+  }
+  if (rc) return library_error(rc);
+  if (out_arg != Py_None) {
+    Py_INCREF(out_arg);
+    return out_arg;
+  }
+  return THPVariable_Wrap(std::move(out));
 }
 
 // decode(q, kv, scale, num_splits, out, workspace, status) -> out, or None
 PyObject *decode(PyObject *, PyObject *const *a, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
   if (n != 7 || !PyLong_Check(a[3])) Py_RETURN_NONE;
   const long splits = PyLong_AsLong(a[3]);
   if (splits == -1 && PyErr_Occurred()) {
@@ -230,17 +236,22 @@ PyObject *decode(PyObject *, PyObject *const *a, Py_ssize_t n) {
     Py_RETURN_NONE;
   }
   return run_decode(a[0], a[1], a[2], splits, a[4], a[5], a[6], false);
+  END_HANDLE_TH_ERRORS
 }
 
 // attend(q, kv, scale, status) -> (B, 1, Hq, D), the layout attention interfaces hand back, or None
 PyObject *attend(PyObject *, PyObject *const *a, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
   if (n != 4) Py_RETURN_NONE;
   return run_decode(a[0], a[1], a[2], 0, Py_None, Py_None, a[3], true);
+  END_HANDLE_TH_ERRORS
 }
 
 // append(k, v, k_pages, k_norms, v_pages, v_norms, page_table, seq_lens, k_tq, v_tq, order, status) -> True, or None
 PyObject *append(PyObject *, PyObject *const *a, Py_ssize_t n) {
-  at::Tensor k, v, kp, kn, vp, vn, table, lens;
+  HANDLE_TH_ERRORS
+  at::Tensor k, v, kp, kn, vp, vn, table, lens, status_tensor;
+  Quant k_quant, v_quant;
   if (n != 12 || !tensor(a[0], k) || !tensor(a[1], v) || !tensor(a[2], kp) || !tensor(a[3], kn) || !tensor(a[4], vp) ||
       !tensor(a[5], vn) || !tensor(a[6], table) || !tensor(a[7], lens))
     Py_RETURN_NONE;
@@ -252,13 +263,13 @@ PyObject *append(PyObject *, PyObject *const *a, Py_ssize_t n) {
   const int64_t B = k.size(0), Hkv = k.size(1), tokens = k.size(2), D = k.size(3);
   if (dtype < 0 || B < 1 || Hkv < 1 || tokens < 1 || D < 1 || D > 256) Py_RETURN_NONE;
   wtq_side_t sk, sv;
-  int64_t bw_k = 0, bw_v = 0;
   int32_t *status;
   sk.centroids = sv.centroids = nullptr;
   if (kp.device() != dev || kn.device() != dev || vp.device() != dev || vn.device() != dev ||
-      !table_and_lengths(table, lens, B, dev) || !quant_table(a[8], N.boundaries, D, 1, dev, bw_k, sk.Pi, sk.bounds) ||
-      !quant_table(a[9], N.boundaries, D, 1, dev, bw_v, sv.Pi, sv.bounds) || !side_pages(kp, kn, bw_k, D, sk) ||
-      !side_pages(vp, vn, bw_v, D, sv) || !optional_status(a[11], dev, status) || kp.size(1) != Hkv || table.size(1) < 1)
+      !table_and_lengths(table, lens, B, dev) || !quant_table(a[8], N.boundaries, D, 1, dev, k_quant, sk.Pi, sk.bounds) ||
+      !quant_table(a[9], N.boundaries, D, 1, dev, v_quant, sv.Pi, sv.bounds) || !side_pages(kp, kn, k_quant.bw, D, sk) ||
+      !side_pages(vp, vn, v_quant.bw, D, sv) || !optional_status(a[11], dev, status_tensor, status) || kp.size(1) != Hkv ||
+      table.size(1) < 1)
     Py_RETURN_NONE;
   for (int i = 0; i < 3; ++i)
     if (kp.size(i) != vp.size(i)) Py_RETURN_NONE;
@@ -279,11 +290,14 @@ PyObject *append(PyObject *, PyObject *const *a, Py_ssize_t n) {
   }
   if (rc) return library_error(rc);
   Py_RETURN_TRUE;
+  END_HANDLE_TH_ERRORS
 }
 
 // stage(dst, src, dst, src, dst, src) -> True, or None: copies of contiguous tensors of equal type and size
 // (a pair of None: nothing to copy)
 PyObject *stage(PyObject *, PyObject *const *a, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  at::Tensor held[3][2];
   void *dst[3] = {};
   const void *src[3] = {};
   int64_t bytes[3] = {};
@@ -291,13 +305,13 @@ PyObject *stage(PyObject *, PyObject *const *a, Py_ssize_t n) {
   if (n != 6) Py_RETURN_NONE;
   for (int i = 0; i < 3; ++i) {
     if (a[2 * i + 1] == Py_None) continue;
-    at::Tensor d, s;
+    at::Tensor &d = held[i][0], &s = held[i][1];
     if (!tensor(a[2 * i], d) || !tensor(a[2 * i + 1], s) || !d.is_cuda() || s.device() != d.device() ||
         d.scalar_type() != s.scalar_type() || d.sizes() != s.sizes() || !d.is_contiguous() || !s.is_contiguous() ||
         (dev.is_cuda() && dev != d.device()))
       Py_RETURN_NONE;
     dev = d.device();
-    dst[i] = d.data_ptr();
+    dst[i] = d.mutable_data_ptr();
     src[i] = s.const_data_ptr();
     bytes[i] = (int64_t)d.nbytes();
     if ((((uintptr_t)dst[i] | (uintptr_t)src[i]) & 15) != 0) Py_RETURN_NONE;
@@ -312,6 +326,7 @@ PyObject *stage(PyObject *, PyObject *const *a, Py_ssize_t n) {
   }
   if (rc) return library_error(rc);
   Py_RETURN_TRUE;
+  END_HANDLE_TH_ERRORS
 }
 
 PyObject *set_error(PyObject *, PyObject *type) {
