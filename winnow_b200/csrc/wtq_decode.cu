@@ -92,7 +92,8 @@ __global__ void __launch_bounds__(kRotThreads) rotate_q_kernel(
     qs[r][d] = v;
   }
   __syncthreads();
-  // the page scan that follows may start its own prologue now
+  // the page scan that follows may start its own prologue now (never before
+  // begin_rotation(): it reads pages and lengths ahead of its wait)
   asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   constexpr int kWarps = kRotThreads / 32, kBatch = 8;

@@ -178,11 +178,12 @@ decode_mma_kernel(DecodeParams p, int chunk_tokens) {
   auto prefix_at = [&](int i) -> int {
     return prefix_local ? (int)lds32(kPrefixAddr + 4 * i) : p.chunk_prefix[i];
   };
-  // The prefix in global memory, q_rot and the tables are written by the
-  // rotation kernel launched just before this one; pages, page table and
-  // lengths are older than that kernel's start (it is launched without the
-  // programmatic attribute), so the first window may be requested before the
-  // wait whenever the prefix is local.
+  // The prefix in global memory, q_rot and the tables are written by the rotation
+  // kernel launched just before this one.  Pages, page table and lengths are complete
+  // when this kernel starts, because every block of the rotation passes its own
+  // griddepcontrol.wait (everything ahead of it has then completed) before any lets this
+  // kernel in; so the first window may be requested before the wait whenever the prefix
+  // is local.
   if (!prefix_local) griddep_wait();
 
   // Items (one chunk of one kv head of one sequence; only chunks that exist are
@@ -466,8 +467,8 @@ __global__ void __launch_bounds__(kMergeThreads, 1) merge_group_kernel(
     }
   }
   asm volatile("griddepcontrol.wait;\n" ::: "memory");      // partial states are complete
-  // (the exchange's wait kernel, if it follows, may be scheduled now: it waits
-  // for this grid to finish before it reads anything)
+  // (the exchange's wait kernel, if it follows, may be scheduled now: it polls flags
+  // that this grid sets last, and ends only after this grid has)
   asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
   if (p.work_counter != nullptr && blockIdx.x == 0 && blockIdx.y == 0 && tid == 0)
     *p.work_counter = 0;
@@ -662,8 +663,8 @@ __global__ void __launch_bounds__(128, 8) merge_small_kernel(MergeParams p, cons
   L = L < 0 ? 0 : (L > max_tokens ? max_tokens : L);
   const int chunks = (L + chunk_tokens - 1) / chunk_tokens;
   asm volatile("griddepcontrol.wait;\n" ::: "memory");      // partial states are complete
-  // (the exchange's wait kernel, if it follows, may be scheduled now: it waits
-  // for this grid to finish before it reads anything)
+  // (the exchange's wait kernel, if it follows, may be scheduled now: it polls flags
+  // that this grid sets last, and ends only after this grid has)
   asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
   if (p.work_counter != nullptr && group == 0 && blockIdx.y == 0 && tid == 0) *p.work_counter = 0;
   const uint32_t exchange_step = p.world > 0 ? *p.step_counter + 1u : 0u;
@@ -741,7 +742,8 @@ __global__ void __launch_bounds__(128, 8) merge_small_kernel(MergeParams p, cons
 // per call}.  The kernel numbers its own calls (state[1]), so it does not
 // depend on the merge kernel ahead of it and starts polling as soon as it is
 // scheduled; the blocks per call are read inside the loop because the local
-// merge may not have recorded them yet.
+// merge may not have recorded them yet.  It ends after the merge does even where its
+// polls run out: what follows in the stream may overwrite the states the merge reads.
 __global__ void exchange_wait_kernel(const uint32_t *flags, int world, uint32_t *state,
                                      long long spin_limit, int32_t *status) {
   const int r = threadIdx.x;
@@ -762,6 +764,7 @@ __global__ void exchange_wait_kernel(const uint32_t *flags, int world, uint32_t 
     }
     if (!arrived && status != nullptr) atomicOr(status, WTQ_STATUS_EXCHANGE_TIMEOUT);
   }
+  griddep_wait();
   __threadfence_system();
 }
 
