@@ -312,6 +312,13 @@ int wtq_dequant_mode(const uint8_t *packed, const void *norms_f16, const float *
 int wtq_dequant_pair(const uint8_t *const packed[2], const void *const norms_f16[2],
                      const float *centroids, const float *Pi, void *const out[2], int out_dtype,
                      int bw, int D, int64_t N, int64_t L, int64_t MAXLEN, void *stream);
+/* The tcgen05 kernel's waits are bounded.  One that runs out leaves rows unwritten; the next
+ * dequantisation call on that device then fails with WTQ_ERR_CUDA, or, asked for after a
+ * synchronisation, wtq_dequant_gave_up returns 1 (either way once).
+ * wtq_dequant_wait_tries: polls after which a wait of this thread's later calls gives up
+ * (0: at once; negative: the default, 2^20), for testing that report. */
+int wtq_dequant_gave_up(void);
+void wtq_dequant_wait_tries(int tries);
 
 /* Instrumentation; no counterpart in the reference.
  * wtq_launch_count: kernels this library has launched in this process.

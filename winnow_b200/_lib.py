@@ -107,6 +107,8 @@ _SIGNATURES = {
     "wtq_dequant_pair": (c_int, [ctypes.POINTER(c_void_p), ctypes.POINTER(c_void_p), c_void_p, c_void_p,
                                  ctypes.POINTER(c_void_p), c_int, c_int, c_int, c_int64, c_int64, c_int64,
                                  c_void_p]),
+    "wtq_dequant_gave_up": (c_int, []),
+    "wtq_dequant_wait_tries": (None, [c_int]),
 }
 
 _lib = None

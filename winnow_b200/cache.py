@@ -346,6 +346,16 @@ class TQPackedLayer(_LayerBase):
         self._len += n
         return self._load_both(self._len)
 
+    def check(self) -> None:
+        """Raise `BackendError` if a reconstruction gave up waiting for the tensor cores
+        and left rows unwritten.  Synchronises; `update` reports an earlier step's
+        without waiting."""
+        if self.is_initialized:
+            with torch.cuda.device(self.device):
+                torch.cuda.current_stream().synchronize()
+                if _lib.lib().wtq_dequant_gave_up():
+                    raise _lib.BackendError("a reconstruction gave up waiting for the tensor cores")
+
     # ---- cache protocol ----------------------------------------------------------
     def get_seq_length(self, *args, **kwargs) -> int:
         return self._len
@@ -413,6 +423,10 @@ class TQPackedCache(_CacheBase):
 
     def update(self, key_states, value_states, layer_idx: int, *args, **kwargs):
         return self.layers[layer_idx].update(key_states, value_states)
+
+    def check(self) -> None:
+        for layer in self.layers:
+            layer.check()
 
     def get_seq_length(self, layer_idx: int = 0, *args, **kwargs) -> int:
         return self.layers[layer_idx].get_seq_length()

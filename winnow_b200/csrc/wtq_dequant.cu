@@ -651,7 +651,17 @@ int launch_exact(const DequantParams &p, cudaStream_t stream) {
   return check_cuda(cudaGetLastError(), "wtq_dequant launch");
 }
 
+// A kernel whose waits ran out left rows unwritten; the next call says so.
+int earlier_call() {
+  if (!dequant_umma_gave_up()) return WTQ_OK;
+  return fail(WTQ_ERR_CUDA, "wtq_dequant: an earlier call on this device gave up waiting for the tensor cores and "
+              "left rows unwritten");
+}
+
 }  // namespace
+
+extern "C" int wtq_dequant_gave_up(void) { return dequant_umma_gave_up() ? 1 : 0; }
+extern "C" void wtq_dequant_wait_tries(int tries) { dequant_umma_wait_tries(tries); }
 
 extern "C" int wtq_dequant_mode(const uint8_t *packed, const void *norms_f16, const float *centroids,
                                 const float *Pi, void *out, int out_dtype, int bw, int D, int64_t N,
@@ -668,6 +678,7 @@ extern "C" int wtq_dequant_mode(const uint8_t *packed, const void *norms_f16, co
   if (L < 1 || MAXLEN < L) return fail(WTQ_ERR_ARG, "wtq_dequant: need 1 <= L <= MAXLEN");
   if (!packed || !norms_f16 || !centroids || !Pi || !out)
     return fail(WTQ_ERR_ARG, "wtq_dequant: null buffer");
+  if (int rc = earlier_call()) return rc;
   DequantParams p;
   p.packed = packed; p.norms = (const __half *)norms_f16; p.centroids = centroids; p.Pi = Pi;
   p.out = out; p.out_dtype = out_dtype; p.bw = bw; p.D = D; p.nb = D * bw / 8;
@@ -708,6 +719,7 @@ extern "C" int wtq_dequant_pair(const uint8_t *const packed[2], const void *cons
                                 const float *centroids, const float *Pi, void *const out[2], int out_dtype,
                                 int bw, int D, int64_t N, int64_t L, int64_t MAXLEN, void *stream_) {
   if (!packed || !norms_f16 || !out) return fail(WTQ_ERR_ARG, "wtq_dequant: null buffer");
+  if (int rc = earlier_call()) return rc;
   const bool complete = packed[0] && packed[1] && norms_f16[0] && norms_f16[1] && out[0] && out[1] && centroids && Pi;
   if (complete && N > 0 && D == 128 && L >= 1 && MAXLEN >= L && (out_dtype == WTQ_F16 || out_dtype == WTQ_BF16)) {
     DequantParams p[2];

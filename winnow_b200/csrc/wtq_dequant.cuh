@@ -17,11 +17,15 @@ struct DequantParams {
   const uint8_t *packed_b = nullptr;
   const __half *norms_b = nullptr;
   void *out_b = nullptr;
+  int wait_tries = 0;           // set by launch_dequant_umma
 };
 
 // tcgen05 kernel (wtq_dequant_umma.cu); `terms` = 1 or 3.  *usable = false and
 // nothing launched when the kernel cannot serve this call here.
 int launch_dequant_umma(const DequantParams &p, int terms, cudaStream_t stream, bool *usable);
-int dequant_umma_gave_up();
+// Whether a wait ran out in it on the current device since this was last asked.
+bool dequant_umma_gave_up();
+// Polls a wait of the calls of this thread makes before it gives up; negative: the default.
+void dequant_umma_wait_tries(int tries);
 
 }  // namespace wtq

@@ -30,6 +30,7 @@
 #include <cuda.h>
 
 #include <atomic>
+#include <cstring>
 #include <mutex>
 
 #include "wtq_common.cuh"
@@ -59,6 +60,7 @@ constexpr float kOperandScale = 256.f, kResultScale = 1.f / (256.f * 256.f);
 constexpr uint32_t kIdesc = (1u << 4) | ((128u >> 3) << 17) | ((128u >> 4) << 24);
 
 constexpr uint32_t kBox = 32 * 128;
+constexpr int kWaitTries = 1 << 20;               // polls of an mbarrier before a wait gives up (each suspends a while)
 
 template <int BW, int TERMS, int DT> struct Map {
   static constexpr uint32_t kLutBytes = mma::lut_entries(BW) * 256u;
@@ -163,8 +165,8 @@ template <int DT> __device__ __forceinline__ uint32_t pack2(float x, float y) {
   }
 }
 
-// state: word 0 = 1 when the shared-memory layout assumption is broken, word 1 =
-// 1 when a wait for the tensor cores ran out.
+// state (host memory): word 0 = 1 when the shared-memory layout assumption is broken, word
+// 1 = 1 when a wait ran out and rows were left unwritten.
 template <int BW, int TERMS, int DT>
 __global__ void __launch_bounds__(kThreads, 1)
 dequant_umma_kernel(DequantParams p, const __grid_constant__ CUtensorMap out_map,
@@ -257,9 +259,9 @@ dequant_umma_kernel(DequantParams p, const __grid_constant__ CUtensorMap out_map
     return (plane0 + wrap) * p.MAXLEN + (pos - wrap * L32);
   };
   // Bounded wait for completion number `use` (0, 1, ...) of an mbarrier; false if it ran out.
-  auto wait_for = [&](uint32_t bar, int use) -> bool {
+  auto wait_tries = [&](uint32_t bar, int use, int tries) -> bool {
     uint32_t done = 0;
-    for (int spin = 0; spin < (1 << 20) && !done; ++spin) {
+    for (int spin = 0; spin < tries && !done; ++spin) {
       asm volatile(
           "{\n\t.reg .pred q;\n\tmbarrier.try_wait.parity.shared::cta.b64 q, [%1], %2;\n\t"
           "selp.u32 %0, 1, 0, q;\n\t}\n"
@@ -267,6 +269,7 @@ dequant_umma_kernel(DequantParams p, const __grid_constant__ CUtensorMap out_map
     }
     return done != 0;
   };
+  auto wait_for = [&](uint32_t bar, int use) -> bool { return wait_tries(bar, use, p.wait_tries); };
 
   // Tile i of this block uses operand and accumulator i & 1.  What orders the groups:
   //   full[b]  arrives (once per decode warp) when operand b is in tensor memory;
@@ -424,6 +427,8 @@ dequant_umma_kernel(DequantParams p, const __grid_constant__ CUtensorMap out_map
       asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n"
                    ::"r"(kBarDone + 8u * buf) : "memory");
     }
+    // nothing is in flight when the tensor memory is freed, also where the others gave up
+    if (i > 0) wait_tries(kBarDone + 8u * ((i - 1) & 1), (i - 1) >> 1, kWaitTries);
   }
   __syncwarp();
   asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
@@ -436,14 +441,46 @@ dequant_umma_kernel(DequantParams p, const __grid_constant__ CUtensorMap out_map
 
 namespace {
 
-__device__ int32_t g_umma_state[2];
-
 template <int BW, int TERMS, int DT> std::atomic<int> &variant_state(int dev) {
   static std::atomic<int> state[64];
   return state[dev & 63];
 }
 
+// The state words of every device, in pinned host memory so that a kernel which gave up is
+// seen without asking the device.
+std::atomic<int32_t *> g_words{nullptr};
+int32_t *state_words(int dev) {                    // null where there is no memory to be had
+  int32_t *words = g_words.load(std::memory_order_acquire);
+  if (!words) {
+    static std::mutex gate;
+    std::lock_guard<std::mutex> hold(gate);
+    words = g_words.load(std::memory_order_acquire);
+    if (!words) {
+      void *p = nullptr;
+      if (cudaHostAlloc(&p, 64 * 2 * sizeof(int32_t), cudaHostAllocPortable | cudaHostAllocMapped) != cudaSuccess) {
+        cudaGetLastError();
+        return nullptr;
+      }
+      memset(p, 0, 64 * 2 * sizeof(int32_t));
+      words = (int32_t *)p;
+      g_words.store(words, std::memory_order_release);
+    }
+  }
+  return words + 2 * (dev & 63);
+}
+thread_local int t_wait_tries = dq5::kWaitTries;
+
 }  // namespace
+
+bool dequant_umma_gave_up() {
+  int32_t *words = g_words.load(std::memory_order_acquire);
+  if (!words) return false;
+  int dev = 0;
+  cudaGetDevice(&dev);
+  words += 2 * (dev & 63) + 1;
+  return __atomic_load_n(words, __ATOMIC_RELAXED) && __atomic_exchange_n(words, 0, __ATOMIC_ACQ_REL);
+}
+void dequant_umma_wait_tries(int tries) { t_wait_tries = tries < 0 ? dq5::kWaitTries : tries; }
 
 // Tensor map of an output, (N, 128) elements, boxes of 32 rows x 128 bytes; false where the
 // driver has no such call or refuses the tensor.
@@ -482,9 +519,6 @@ static int launch_variant(const DequantParams &p, cudaStream_t stream, bool *usa
   int dev = 0;
   cudaGetDevice(&dev);
   std::atomic<int> &state = variant_state<BW, TERMS, DT>(dev);
-  int32_t *flag = nullptr;
-  if (cudaGetSymbolAddress((void **)&flag, g_umma_state) != cudaSuccess)
-    return check_cuda(cudaGetLastError(), "wtq_dequant: tensor-memory kernel set-up");
   auto kernel = dq5::dequant_umma_kernel<BW, TERMS, DT>;
   int s = state.load(std::memory_order_acquire);
   if (s == 0) {
@@ -494,10 +528,10 @@ static int launch_variant(const DequantParams &p, cudaStream_t stream, bool *usa
     static std::mutex gate;
     std::lock_guard<std::mutex> hold(gate);
     if ((s = state.load(std::memory_order_acquire)) == 0) {
+      int32_t *const flag = state_words(dev);
+      if (!flag) return WTQ_OK;
       cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                            (int)M::kDynamic);
-      int32_t seen[2] = {0, 0};
-      if (e == cudaSuccess) e = cudaMemsetAsync(flag, 0, sizeof(seen), stream);
       if (e == cudaSuccess) {
         DequantParams none = {};
         none.L = none.MAXLEN = 1;
@@ -505,10 +539,9 @@ static int launch_variant(const DequantParams &p, cudaStream_t stream, bool *usa
         note_launches(1);
         e = cudaGetLastError();
       }
-      if (e == cudaSuccess) e = cudaMemcpyAsync(seen, flag, sizeof(seen), cudaMemcpyDeviceToHost, stream);
       if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
       if (e != cudaSuccess) return check_cuda(e, "wtq_dequant: tensor-memory kernel set-up");
-      s = seen[0] ? 2 : 1;
+      s = __atomic_load_n(flag, __ATOMIC_ACQUIRE) ? 2 : 1;
       state.store(s, std::memory_order_release);
     }
   }
@@ -528,7 +561,9 @@ static int launch_variant(const DequantParams &p, cudaStream_t stream, bool *usa
   cfg.stream = stream;
   cfg.attrs = &pdl;
   cfg.numAttrs = 1;
-  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, p, map, map_b, flag);
+  DequantParams job = p;
+  job.wait_tries = t_wait_tries;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, job, map, map_b, state_words(dev));
   note_launches(1);
   *usable = true;
   return check_cuda(e, "wtq_dequant tensor-memory launch");
@@ -550,14 +585,6 @@ int launch_dequant_umma(const DequantParams &p, int terms, cudaStream_t stream, 
   if (p.bw == 4) return launch_dtype<4, 1>(p, stream, usable);
   if (p.bw == 6) return launch_dtype<6, 1>(p, stream, usable);
   return launch_dtype<8, 1>(p, stream, usable);
-}
-
-// 1 if a wait for the tensor cores ran out in a tcgen05 dequantisation kernel
-// since the library was loaded (synchronises the device; a diagnostic).
-int dequant_umma_gave_up() {
-  int32_t seen[2] = {0, 0};
-  if (cudaMemcpyFromSymbol(seen, g_umma_state, sizeof(seen)) != cudaSuccess) return -1;
-  return seen[1];
 }
 
 }  // namespace wtq
