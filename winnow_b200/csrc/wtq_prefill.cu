@@ -63,6 +63,7 @@ constexpr uint32_t kPFull = kBase + 96;             // [M tile][buffer]: probabi
 constexpr uint32_t kODone = kBase + 128;            // [M tile][buffer]: the products of a tile into O are complete
 constexpr uint32_t kTmemSlot = kBase + 160;         // tensor-memory address written by tcgen05.alloc
 constexpr uint32_t kAbort = kBase + 164;            // a wait ran out
+constexpr uint32_t kLast = kBase + 168;             // everything issued is complete
 constexpr uint32_t kItem = kBase + 176;             // the item being worked on (8 words)
 constexpr uint32_t kWalk = kItem + 32;              // balanced schedule: where this block stands (10 words)
 constexpr uint32_t kTileBytes = kTile * 256;        // a decoded tile: [64 tokens][128] fp16
@@ -158,16 +159,20 @@ __device__ __forceinline__ uint32_t elect_one() {
   asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}\n" : "=r"(r));
   return r;
 }
+constexpr int kWaitTries = 1 << 20;
+__device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
+  uint32_t done;
+  asm volatile(
+      "{\n\t.reg .pred q;\n\tmbarrier.try_wait.parity.shared::cta.b64 q, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, q;\n\t}\n"
+      : "=r"(done) : "r"(bar), "r"(parity) : "memory");
+  return done != 0;
+}
 // Bounded wait for completion number `use` (0, 1, ..) of an mbarrier; false if it, or any
 // other wait of the block, ran out.
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, int use) {
-  for (int spin = 0; spin < (1 << 20); ++spin) {
-    uint32_t done;
-    asm volatile(
-        "{\n\t.reg .pred q;\n\tmbarrier.try_wait.parity.shared::cta.b64 q, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, q;\n\t}\n"
-        : "=r"(done) : "r"(bar), "r"((uint32_t)(use & 1)) : "memory");
-    if (done) return true;
+  for (int spin = 0; spin < kWaitTries; ++spin) {
+    if (mbar_try(bar, (uint32_t)(use & 1))) return true;
     if ((spin & 255) == 255 && lds32(kAbort) != 0u) return false;
   }
   sts32(kAbort, 0x80000000u | (threadIdx.x >> 5) << 24 | ((uint32_t)use & 0xfffu) << 12 | (bar - kBase));   // who gave up on what
@@ -368,6 +373,7 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_kernel(Params p) {
       mbar_init(kODone + 8u * i, 1);
       mbar_init(kPFull + 8u * i, 4);                        // the four warps of an M tile
     }
+    mbar_init(kLast, 1);
     sts32(kAbort, 0u);
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
   }
@@ -777,8 +783,17 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_kernel(Params p) {
     p.work_counter[1] = (int)lds32(kAbort);                 // (for whoever looks into the workspace)
     if (p.status) atomicOr(p.status, WTQ_STATUS_SCAN_TIMEOUT);
   }
-  if (warp == kMmaWarp)
+  if (warp == kMmaWarp) {
+    // A block that gave up may have products in flight: they end before their tensor memory
+    // goes to somebody else (bounded, like every wait).
+    fence_after();
+    if (elect_one()) umma_commit(kLast);
+    __syncwarp();
+    for (int spin = 0; spin < kWaitTries && !mbar_try(kLast, 0u); ++spin) {
+    }
+    __syncwarp();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(kCols) : "memory");
+  }
 }
 
 template <int BWK, int BWV>
