@@ -607,10 +607,12 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_kernel(Params p) {
         float sa = 0.f, sb = 0.f;
 #pragma unroll
         for (int i = 0; i < 32; ++i) {
-          const float x = ex2(__uint_as_float(s[2 * i]) - base), y = ex2(__uint_as_float(s[2 * i + 1]) - base);
-          sa += x;
-          sb += y;
-          pr[i] = pack_half2(x, y);
+          pr[i] = pack_half2(ex2(__uint_as_float(s[2 * i]) - base), ex2(__uint_as_float(s[2 * i + 1]) - base));
+          // The sum takes the probabilities as the product has them: where a few keys carry the
+          // row, their rounding then cancels in the quotient.
+          const float2 pq = __half22float2(*reinterpret_cast<const __half2 *>(&pr[i]));
+          sa += pq.x;
+          sb += pq.y;
         }
         sum += sa + sb;
         tmem_store32(s_addr, pr);                                       // over the scores just read
