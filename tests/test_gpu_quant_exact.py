@@ -31,6 +31,14 @@ def test_vector_counts_and_types(rows, dtype):
     check(x.to(dtype), 4)
 
 
+@pytest.mark.parametrize("rows", [443, 444, 445, 447, 449, 464, 465, 592, 593])
+def test_where_the_tensor_cores_take_over(rows):
+    """Three vectors a multiprocessor (444 at 148), and the passes of 16 just above."""
+    x = torch.randn(rows, 128, generator=torch.Generator().manual_seed(rows)).half()
+    for bw in (3, 4, 8):
+        check(x, bw)
+
+
 @pytest.mark.parametrize("bw", [2, 3, 4, 5, 6, 8])
 def test_widths_and_special_rows(bw):
     x = torch.randn(3000, 128, generator=torch.Generator().manual_seed(bw))

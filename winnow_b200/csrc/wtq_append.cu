@@ -474,7 +474,9 @@ extern "C" int wtq_quantize(const void *x, int dtype, int64_t rows, int64_t row_
   a.vec_dst = ((uintptr_t)idx & 7) == 0 && ((uintptr_t)packed & 7) == 0;
   a.pages = packed; a.idx = idx; a.norms32 = norms;
   job.vectors = rows; job.dtype = dtype;
-  if (quant_mma_eligible(D, p.order, job, 1))
+  // Up to three vectors a multiprocessor run at once with a block each: 6 / 64 / 256 rows 6.7 /
+  // 6.7 / 8.4 us, 9.3 / 10.8 / 12.3 on the tensor cores, which take 12.9 at 512 (14.9 here).
+  if (rows > 3 * (int64_t)device_sms() && quant_mma_eligible(D, p.order, job, 1))
     return launch_quant_mma(job, false, 1, (cudaStream_t)stream, "wtq_quantize launch");
   return launch_staged(quantize_kernel<true>, quantize_kernel<false>, p, D, rows, 1,
                        (cudaStream_t)stream, "wtq_quantize launch");
