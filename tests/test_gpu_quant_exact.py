@@ -48,6 +48,19 @@ def test_widths_and_special_rows(bw):
     check(x, bw)
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("bw", [2, 4, 6, 8])
+def test_zero_vectors_among_others(bw, dtype):
+    """Vectors of zeros (of either sign) sit on the middle boundary exactly; vectors whose
+    squares vanish, or with one element only, do not."""
+    x = torch.randn(1200, 128, generator=torch.Generator().manual_seed(bw))
+    x[::3] = 0.0
+    x[3::9] = -0.0
+    x[600:900] = 0.0                                    # whole passes
+    x[601, 5], x[607, 127], x[613], x[640, 0] = 1e-23, -1e-30, 1e-25, 2.0
+    check(x.to(dtype), bw)
+
+
 def on_boundaries(bw):
     oq = orc.OracleQuantizer.get(bw, 128, 42)
     g = torch.Generator().manual_seed(99)

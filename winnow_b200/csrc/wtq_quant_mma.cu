@@ -240,7 +240,7 @@ __global__ void __launch_bounds__(kThreads, 1) quant_mma_kernel(QuantJob job) {
     }
     // ---- rows g and g + 8: norm, division, A fragments ---------------------------------
     uint32_t ah[8][4], al[8][4];
-    float norm[2];
+    float norm[2], near_by[2];                                    // near_by: how near a boundary asks for the chain
     float2 x[2][16];
 #pragma unroll
     for (int r = 0; r < 2; ++r) {
@@ -263,6 +263,15 @@ __global__ void __launch_bounds__(kThreads, 1) quant_mma_kernel(QuantJob job) {
         total = __fadd_rn(total, __shfl_sync(kFull, s1, (lane & 28) + k));
       }
       norm[r] = fmaxf(__fsqrt_rn(total), 1e-10f);
+      near_by[r] = margin;
+      // A vector of zeros (padding) gives y = y' = 0 exactly, and a boundary is often there:
+      // no chains for it.  (A NaN among the products still fails the comparison.)
+      if (__any_sync(kFull, total == 0.f)) {
+        bool zero = total == 0.f;
+#pragma unroll
+        for (int m = 0; m < 16; ++m) zero = zero && x[r][m].x == 0.f && x[r][m].y == 0.f;
+        if ((__ballot_sync(kFull, zero) >> (lane & 28) & 15u) == 15u) near_by[r] = -1.f;
+      }
     }
 #pragma unroll
     for (int r = 0; r < 2; ++r)
@@ -305,7 +314,7 @@ __global__ void __launch_bounds__(kThreads, 1) quant_mma_kernel(QuantJob job) {
           k[e] = bucket(s, nbounds, y);
           edge = s.around[k[e]];
         }
-        doubt[e] = !(y - edge.x > margin) || !(edge.y - y > margin);
+        doubt[e] = !(y - edge.x > near_by[(e >> 1) & 1]) || !(edge.y - y > near_by[(e >> 1) & 1]);
       }
 #pragma unroll
       for (int e = 0; e < 8; e += 2)                             // rows g, g + 8; coordinates 2t, 2t + 1
