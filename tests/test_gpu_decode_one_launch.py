@@ -59,3 +59,24 @@ def test_refused_pages_and_positions_are_reported():
     out = packed_decode_attention(q.cuda(), kv, orc.default_scale(c.D), check_page_ids=False, status=status)
     assert int(status.item()) == _lib.STATUS_BAD_PAGE | _lib.STATUS_BAD_POSITION
     assert torch.isfinite(out).all()
+
+
+@pytest.mark.parametrize("B,Hq,Hkv,widths,width_tokens,launches", [
+    (18, 32, 8, (4, 4), 131072, 3), (16, 32, 8, (4, 4), 8192, 3), (16, 32, 8, (4, 4), 2048, 1),
+    (32, 28, 4, (8, 8), 1984, 1), (32, 28, 4, (8, 8), 4096, 3), (16, 32, 8, (6, 6), 2048, 3), (16, 32, 8, (4, 6), 4096, 3),
+    (4, 32, 8, (4, 4), 65536, 3), (8, 32, 8, (4, 4), 8192, 3), (1, 32, 8, (4, 4), 16384, 1), (1, 32, 8, (4, 4), 131072, 3)])
+def test_long_tables_go_to_the_whole_chip(B, Hq, Hkv, widths, width_tokens, launches):
+    """One launch lasts as long as the longest sequence may be: tables that admit one which
+    the split-K path would share out go there, with the same result either way."""
+    c = C("width", 60, B, Hq, Hkv, 128, (300,) + (40,) * (B - 1), 16, *widths)
+    q, okv, _ = oracle_case(c)
+    kv = to_device(okv, "cuda")
+    wide = torch.full((B, width_tokens // 16), -1, dtype=torch.int32, device="cuda")
+    wide[:, :kv.page_table.shape[1]] = kv.page_table
+    kv.page_table = wide
+    q, scale = q.cuda(), orc.default_scale(128)
+    packed_decode_attention(q, kv, scale, check_page_ids=False)
+    before = _lib.lib().wtq_launch_count()
+    got = packed_decode_attention(q, kv, scale, check_page_ids=False)
+    assert _lib.lib().wtq_launch_count() - before == launches
+    assert_attention_close(got, packed_decode_attention(q, kv, scale, num_splits=2, check_page_ids=False))

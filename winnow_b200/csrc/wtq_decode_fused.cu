@@ -510,13 +510,24 @@ template <int D> int launch_widths(const Params &p, int B, int Hkv, int cluster,
 // more than it brings (32 groups of 8192 tokens: 22.4 us with 4, 49 with 8), and
 // 16 was never better than 8.
 //
-// At head_dim 128 one launch takes about 10 us + 4.6 ns x tokens / c, the three
-// launches of the split-K path 17.5 us + 4.9 ns x tokens x groups / SMs (4-bit
-// codes; wider ones in proportion to what a token costs to decode), so one launch
-// wins up to 8192 tokens at 128 groups (49.3 against 53.0 us) and 16k at 8 groups
-// (21.2 against 22.5), and loses where it cannot fill the chip (8 groups of 131072
-// tokens: 89 against 55).  With more groups than multiprocessors it would repeat
-// its set-up in every round (320 groups of 1000 tokens: 47.7 against 41.5).
+// At head_dim 128 the table's width says how long a sequence may be, not how long the others
+// are, and the two paths depend on that differently: one launch lasts as long as its longest
+// group, `one` ns a token over the cluster's blocks; the split-K path deals chunks of all
+// groups to the whole chip.  The line is drawn at the mix that favours split-K most, one
+// sequence of the full width among short ones, for which its chunks still cost `split` ns a
+// token x groups / multiprocessors: one launch where it saves more in fixed costs (`gap` us)
+// than it then loses.  Measured (page pools in turn, larger than L2), one launch / split-K, us:
+//   4/4 bits, 128 groups, one sequence of 2048 19.0 / 22.0, of 4096 28.4 / 27.1 (all of 4096
+//   31.8 / 38.5), of 8192 47.5 / 37.1 (all 50.4 / 54.1); 64 groups 4096 19.8 / 21.8, 8192 29.6 / 27.2;
+//   32 groups 8192 21.9 / 23.9, 16384 32.2 / 29.1; 144 groups 131072 575 / 66;
+//   8/8 bits, 128 groups 2048 27.4 / 30.3, 4096 46.9 / 39.6; 32 groups 4096 20.8 / 23.3, 8192 31.3 / 29.7;
+//   6/6 bits, 128 groups 1024 17.6 / 23.0, 2048 26.1 / 24.9; 64 groups 2048 18.1 / 22.7, 4096 27.2 / 25.2;
+//   4/6 bits, 128 groups 2048 22.7 / 25.7, 4096 35.9 / 32.2; 64 groups 4096 23.8 / 25.4, 8192 36.7 / 31.8.
+// One sequence alone has no others: its equal groups cost split-K 4.9 ns a token x groups /
+// multiprocessors (times what a token of these widths costs to decode): 8 groups of 16384 21.4 /
+// 24.0, of 32768 28.0 / 27.6, of 131072 89 / 55.
+// With more groups than multiprocessors one launch would repeat its set-up in every round (320
+// groups of 1000 tokens: 47.7 against 41.5).
 int fused_cluster(const DecodeParams &p) {
   const int64_t groups = (int64_t)p.B * p.Hkv, sms = device_sms();
   const int64_t tokens = (int64_t)p.max_pages * p.S, windows = (tokens + kIterTokens - 1) / kIterTokens;
@@ -526,8 +537,18 @@ int fused_cluster(const DecodeParams &p) {
   for (int i = 1; i < 4 && groups <= ready->clusters[i] && windows >= 4 << i; ++i) c = 1 << i;
   if (p.D == 64) return c;                  // (the alternative is the CUDA-core path)
   if (groups > sms) return 0;
-  const double width = (p.k.bw + p.v.bw) / 8.0 * (p.k.bw + p.v.bw > 8 ? 1.25 : 1.0);
-  return width * (double)tokens * (4.6 / c - 4.9 * (double)groups / (double)sms) <= 7500.0 ? c : 0;
+  const double share = (double)groups / (double)sms;
+  if (p.B == 1) {
+    const double width = (p.k.bw + p.v.bw) / 8.0 * (p.k.bw + p.v.bw > 8 ? 1.25 : 1.0);
+    return width * (double)tokens * (4.6 / c - 4.9 * share) <= 7500.0 ? c : 0;
+  }
+  struct Costs {
+    double one, split, gap;
+  };
+  const Costs w = p.v.bw == 4 ? Costs{4.65, 2.8, 6.3} : p.k.bw == 4 ? Costs{6.4, 3.35, 8.0}
+                  : p.k.bw == 6 ? Costs{7.9, 4.05, 7.0} : Costs{9.2, 5.4, 9.5};
+  const double one = w.one / c * (c >= 4 ? 1.18 : 1.0);       // (short shares of a block: 32-token windows)
+  return (double)tokens * (one - w.split * share) <= 1000.0 * w.gap ? c : 0;
 }
 
 bool fused_eligible(const DecodeParams &p) {
