@@ -291,9 +291,19 @@ def test_append_then_decode_through_the_cache():
     assert_attention_close(out.transpose(1, 2), orc.tiled_attention(q, okv, D ** -0.5))
 
 
-def test_repeated_calls_reuse_the_marshalled_plan():
-    """Same buffers, page ids vouched for: the second call takes the remembered
-    plan, sees data updated in place, and still matches the oracle."""
+class _SlottedKV:
+    """A layer's pages without `PackedKV` (and without weak references)."""
+    __slots__ = ("k_pages", "k_norms", "v_pages", "v_norms", "page_table", "seq_lens", "k_quant", "v_quant",
+                 "head_dim")
+
+    def __init__(self, kv):
+        for name in self.__slots__:
+            setattr(self, name, getattr(kv, name))
+
+
+def test_repeated_calls_see_what_changed():
+    """Same buffers again and again, page ids vouched for: every call reads query, lengths,
+    table and pages as they are then, returns `out`, and keeps nothing of an earlier one."""
     from winnow_b200 import packed_attention_cuda as pac
     c = cases.AttnCase("plan", 31, 2, 8, 2, 128, (70, 33), 16, 4, 4)
     q, okv, _ = oracle_case(c)
@@ -302,18 +312,31 @@ def test_repeated_calls_reuse_the_marshalled_plan():
     qd = q.to(DEV)
     out = torch.empty_like(qd)
     ws = pac.decode_workspace(2, 8, 2, 128, kv.page_table.shape[1], 16, 0, DEV)
-    pac._PLANS.clear()
-    first = packed_decode_attention(qd, kv, scale, out=out, workspace=ws, check_page_ids=False).clone()
-    assert len(pac._PLANS) == 1
+
+    def call(layer, into):
+        got = packed_decode_attention(qd, layer, scale, out=into, workspace=ws, check_page_ids=False)
+        assert got is into
+        return got.clone()
+
+    assert_attention_close(call(kv, out), orc.tiled_attention(q, okv, scale))
     q2 = torch.randn(q.shape, generator=torch.Generator().manual_seed(5))
     qd.copy_(q2)                                         # new query, same buffer
-    second = packed_decode_attention(qd, kv, scale, out=out, workspace=ws, check_page_ids=False)
-    assert len(pac._PLANS) == 1 and second.data_ptr() == out.data_ptr()
-    assert_attention_close(first, orc.tiled_attention(q, okv, scale))
-    assert_attention_close(second, orc.tiled_attention(q2, okv, scale))
-    # a checked call never uses the cache
-    packed_decode_attention(qd, kv, scale, out=out, workspace=ws)
-    assert len(pac._PLANS) == 1
+    assert_attention_close(call(kv, out), orc.tiled_attention(q2, okv, scale))
+    okv.seq_lens.copy_(torch.tensor([41, 20]))           # shorter, and other pages behind the table
+    kv.seq_lens.copy_(okv.seq_lens)
+    okv.page_table[0, :2] = okv.page_table[0, :2].flip(0)
+    kv.page_table.copy_(okv.page_table)
+    okv.v_pages.copy_(okv.v_pages.flip(2))
+    kv.v_pages.copy_(okv.v_pages)
+    ref = orc.tiled_attention(q2, okv, scale)
+    assert_attention_close(call(kv, out), ref)
+    other = torch.empty_like(qd)
+    assert_attention_close(call(kv, other), ref)
+    assert_attention_close(call(_SlottedKV(kv), out), ref)
+    kv.seq_lens = kv.seq_lens + 3                        # a new tensor in the same object
+    okv.seq_lens += 3
+    assert_attention_close(call(kv, out), orc.tiled_attention(q2, okv, scale))
+    assert_attention_close(other, ref)                   # what an earlier call returned stays
 
 
 def test_legacy_contiguous_cache_roundtrip():

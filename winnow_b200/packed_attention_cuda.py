@@ -12,7 +12,6 @@ length.
 from __future__ import annotations
 
 import ctypes
-import weakref
 
 import torch
 
@@ -174,8 +173,6 @@ def packed_decode_attention(q: torch.Tensor, kv: pa.PackedKV, scale: float, *,
     if not check_page_ids:             # checked, allocated for and launched in native code
         got = _lib.host().decode(q, kv, scale, num_splits or 0, out, workspace, status)
         if got is not None:
-            if out is not None and workspace is not None:
-                _remember(q, kv, out, workspace)
             return got
     with torch.no_grad():
         if q.dim() == 4 and q.stride(-1) != 1:
@@ -302,19 +299,3 @@ def dense_decode_attention(q: torch.Tensor, kv: "pa.DenseKV", scale: float, *, n
             ws.data_ptr(), ws.numel(), status.data_ptr() if status is not None else None,
             _lib.stream_ptr(dev)))
     return out
-
-
-# Buffer sets of repeated calls (query, K/V, result and workspace a serving loop
-# updates in place), weakly held: what a caller inspecting the operator sees of its
-# steady state.  The native call reads the tensors anew every time, so an entry is
-# never relied on and may be dropped at any moment.
-_PLANS: dict = {}
-_PLAN_CACHE_SIZE = 256
-
-
-def _remember(q, kv, out, workspace) -> None:
-    key = (id(q), id(kv), id(out), id(workspace))
-    if key not in _PLANS:
-        if len(_PLANS) >= _PLAN_CACHE_SIZE:
-            _PLANS.pop(next(iter(_PLANS)), None)
-        _PLANS[key] = weakref.ref(kv)
