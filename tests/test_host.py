@@ -91,6 +91,18 @@ def test_batch_reservation_and_device_table():
         p.ensure_many(["z"], [4 * 9])                        # beyond the per-request limit
 
 
+def test_layer_views_follow_the_storage():
+    for dense in (None, torch.float32):
+        pool = PagePool(num_layers=2, num_pages=3, num_kv_heads=2, page_size=4, nb_k=8, nb_v=8, dense_dtype=dense)
+        first = pool.layer(1)
+        assert pool.layer(1)[0] is first[0] and (first[1] is None) == (dense is not None)
+        for change in (lambda t: setattr(pool, "v_pages", torch.ones_like(t)), lambda t: t.set_(torch.ones_like(t) * 2),
+                       lambda t: setattr(t, "data", torch.ones_like(t) * 3)):
+            change(pool.v_pages)
+            got = pool.layer(1)[2]
+            assert got.data_ptr() == pool.v_pages[1].data_ptr() and torch.equal(got, pool.v_pages[1])
+
+
 def test_contract_rejections_on_metadata():
     c = cases.ATTENTION_CASES[3]
     q, okv, _ = oracle_case(c)

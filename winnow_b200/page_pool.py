@@ -279,12 +279,14 @@ class PagePool:
 
     def layer(self, index: int):
         """(k_pages, k_norms, v_pages, v_norms) of one layer: views made once per
-        storage (a forward asks for them in every layer)."""
+        storage (a forward asks for them in every layer).  A tensor object may get
+        another storage under it (`set_`, `.data`), so its address counts too."""
         store = (self.k_pages, self.k_norms, self.v_pages, self.v_norms)
-        if self._layers is None or any(a is not b for a, b in zip(self._layers[0], store)):
+        at = [None if t is None else t.data_ptr() for t in store]
+        if self._layers is None or at != self._layers[1] or any(a is not b for a, b in zip(self._layers[0], store)):
             views = [tuple(None if t is None else t[i] for t in store) for i in range(self.num_layers)]
-            self._layers = (store, views)
-        return self._layers[1][index]
+            self._layers = (store, at, views)
+        return self._layers[2][index]
 
 
 class DeviceTable:
