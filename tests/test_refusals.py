@@ -6,8 +6,9 @@ import pytest
 import torch
 from torch._subclasses.fake_tensor import FakeTensorMode
 
-from winnow_b200 import _lib, packed_backend as pb
+from winnow_b200 import _lib, packed_attention as pa, packed_backend as pb
 from winnow_b200.cache import TQPackedLayer
+from winnow_b200.packed_attention_cuda import DecodePlan
 
 
 @pytest.fixture
@@ -36,6 +37,19 @@ def test_append_needs_a_table_row_and_a_length_per_sequence(fake, rows, lens):
 def test_append_needs_its_quantizers_on_the_device(fake):
     with pytest.raises(_lib.BackendError):
         pb.AppendPlan(*_append_args(Pi_device="cpu"))
+
+
+@pytest.mark.parametrize("which", ["workspace", "status"])
+def test_buffers_in_pageable_host_memory(fake, which):
+    args = _append_args()
+    on_host = torch.empty(1 << 20, dtype=torch.uint8 if which == "workspace" else torch.int32, device="cpu")
+    quant = pa.Quantizer.from_tq(args[8])
+    kv = pa.PackedKV(*args[2:8], quant, quant, 128)
+    with pytest.raises(_lib.BackendError, match=which):
+        DecodePlan(torch.empty(4, 8, 1, 128, device="cuda"), kv, 1.0, check_page_ids=False, **{which: on_host})
+    if which == "status":
+        with pytest.raises(_lib.BackendError, match=which):
+            pb.AppendPlan(*args, status=on_host)
 
 
 @pytest.mark.parametrize("k_shape,v_shape", [((3, 2, 8, 128), None), ((1, 2, 8, 128), None), ((8, 2, 8, 128), None),

@@ -175,6 +175,12 @@ def require_cuda(*tensors: torch.Tensor) -> torch.device:
     return dev
 
 
+def reachable(what: str, t: torch.Tensor | None) -> None:
+    """A buffer the kernels write beside their operands: device memory, or pinned host memory."""
+    if t is not None and t.device.type == "cpu" and not t.is_pinned():
+        raise BackendError(f"{what} is in pageable host memory, which the kernels cannot reach")
+
+
 def stream_ptr(device: torch.device) -> int:
     return torch.cuda.current_stream(device).cuda_stream
 

@@ -85,6 +85,8 @@ class DecodePlan:
         elif tuple(out.shape) != (B, Hq, 1, D) or out.dtype != q.dtype or out.stride(-1) != 1 \
                 or out.device != dev:
             raise pa.UnsupportedLayout("out must be (B, Hq, 1, D) in q.dtype with unit stride in D")
+        _lib.reachable("workspace", workspace)
+        _lib.reachable("status", status)
         self.out, self.device = out, dev
         self.empty = B == 0 or max_pages == 0
         if self.empty:

@@ -205,6 +205,7 @@ class AppendPlan:
                  *, order: int = _lib.ORDER_AUTO, status: torch.Tensor | None = None):
         dev = _lib.require_cuda(k, v, k_pages, v_pages, k_norms, v_norms, page_table, seq_lens,
                                 k_tq.Pi, k_tq.boundaries, v_tq.Pi, v_tq.boundaries)
+        _lib.reachable("status", status)
         B, Hkv, n, D = k.shape
         if v.shape != k.shape or v.dtype != k.dtype:
             raise ValueError("k and v must have the same shape and dtype")
