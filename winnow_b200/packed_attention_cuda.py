@@ -187,9 +187,6 @@ def packed_decode_attention(q: torch.Tensor, kv: pa.PackedKV, scale: float, *,
             return plan.run()
 
 
-_PREFILL_WS: dict = {}
-
-
 @torch.no_grad()
 def packed_prefill_attention(q: torch.Tensor, kv: pa.PackedKV, scale: float, *,
                              num_splits: int | None = None, check_page_ids: bool = True,
@@ -220,11 +217,8 @@ def packed_prefill_attention(q: torch.Tensor, kv: pa.PackedKV, scale: float, *,
     asked = max(int(num_splits or 0), 0)                      # 0: the library chooses the schedule
     splits = asked or L.wtq_prefill_auto_splits(B, Hq, Hkv, Q, max_pages, S)
     need = L.wtq_prefill_workspace_bytes(B, Hq, Hkv, Q, D, splits)
-    if workspace is None:
-        key = (dev.index, torch.cuda.current_stream(dev).cuda_stream)
-        workspace = _PREFILL_WS.get(key)
-        if workspace is None or workspace.numel() < need:
-            workspace = _PREFILL_WS[key] = torch.empty(need, dtype=torch.uint8, device=dev)
+    if workspace is None:            # (this call's alone: other threads may be launching on the same stream)
+        workspace = torch.empty(need, dtype=torch.uint8, device=dev)
     k_side = _side(kv.k_pages, kv.k_norms, kv.k_quant)
     v_side = _side(kv.v_pages, kv.v_norms, kv.v_quant)
     with torch.cuda.device(dev):
