@@ -457,7 +457,10 @@ template <int D, int BWK, int BWV> int set_up(const Setup *&out) {
     cfg.numAttrs = 1;
     e = cudaOccupancyMaxActiveClusters(&s.clusters[i], kernel, &cfg);
   }
-  if (e != cudaSuccess) return check_cuda(e, "wtq_decode: fused kernel set-up");
+  if (e != cudaSuccess) {
+    cudaGetLastError();                     // the split-K path serves the call: its launches must not find this error
+    return check_cuda(e, "wtq_decode: fused kernel set-up");
+  }
   s.state.store(1, std::memory_order_release);
   return WTQ_OK;
 }
