@@ -35,33 +35,53 @@
 // mma.sync is the right tensor instruction here: the operands are born in
 // registers; tcgen05 would need them written back to shared memory first.
 //
+// The tile code is this file's own, although wtq_scan.cuh has the same steps for the
+// one-launch kernel: shared through that header the compiler scheduled this kernel 2 %
+// slower (16 x 8 heads x 32768 tokens 137.6 -> 140.5 us, 1 x 8 x 131072 46.0 -> 47.2).
+//
 // Reference schedule being reproduced: turboquant_kv/packed_attention.py:
 // 260-334 (tiled online softmax), split merge :328-334.
 #include <algorithm>
 #include <cstdlib>
-#include <atomic>
+#include <type_traits>
 
-#include "wtq_scan.cuh"
+#include "wtq_decode.cuh"
+#include "wtq_lut.cuh"
+
+#include <atomic>
 
 namespace wtq {
 
 namespace mma {
 
+constexpr int kTileTokens = 16;
+constexpr int kTilesPerIter = 2;                       // 32 tokens per iteration
+constexpr int kIterTokens = kTileTokens * kTilesPerIter;
 constexpr uint32_t kPrefixAddr = 2048;                 // chunk prefix copy (>= dynamic smem base)
 constexpr int kPrefixMax = 1024;                       // entries (sequences + 1) it can hold
 constexpr uint32_t kLutBar = kPrefixAddr + 4 * kPrefixMax;    // mbarrier of the tables' copy
 constexpr uint32_t kFifoAddr = kLutBar + 64;           // per warp: four decoded items of 32 bytes
 constexpr uint32_t kRingLow = kFifoAddr + 16 * 128;    // rings start here
+constexpr uint32_t kSmemLimit = 227 * 1024;
+constexpr float kPreciseAbove = 8.0f;   // |score| (log2 units) that triggers fp32 rescoring
+constexpr float kSlack = 4.0f;          // the softmax reference is set this far above a new maximum
 constexpr int kWaitTries = 1 << 18;     // bound of the mbarrier wait (each try suspends for a while)
 // Worker warps per CTA.  Twelve warps of 168 registers beat sixteen of 128 on
 // every benchmark shape: the lookups of a warp overlap better than more warps do.
 constexpr int kMaxWarps = 12;
 
+constexpr int cmax(int a, int b) { return a > b ? a : b; }
+constexpr int cmin(int a, int b) { return a < b ? a : b; }
+
 // Shared-memory plan of one (key width, value width) instantiation.
-template <int BWK, int BWV>
-struct Cfg : Slot<128, BWK, BWV, BWV == 4 ? 80 : 16 * BWV> {    // (4-bit value rows are padded)
-  using Base = Slot<128, BWK, BWV, BWV == 4 ? 80 : 16 * BWV>;
-  static constexpr int kRing = 2 * kTilesPerIter * Base::kSlot;       // two windows per warp
+template <int BWK, int BWV> struct Cfg {
+  static constexpr int NBK = 16 * BWK, NBV = 16 * BWV;          // bytes per packed row
+  static constexpr int kVRow = BWV == 4 ? 80 : NBV;             // 4-bit value rows are padded
+  static constexpr int kOffV = kTileTokens * NBK;               // tile slot: K | V | nK | nV
+  static constexpr int kOffNK = kOffV + kTileTokens * kVRow;
+  static constexpr int kOffNV = kOffNK + 32;
+  static constexpr int kSlot = kOffNV + 32;
+  static constexpr int kRing = 2 * kTilesPerIter * kSlot;       // two windows per warp
   static constexpr uint32_t kLutBytes = cmax(lut_entries(BWK), lut_entries(BWV)) * 256u;
   static constexpr int kRingsBelow = (int)((kLutAddr - kRingLow) / kRing);
   static constexpr int kRingsAbove = (int)((kSmemLimit - kLutAddr - kLutBytes) / kRing);
@@ -77,6 +97,15 @@ struct Cfg : Slot<128, BWK, BWV, BWV == 4 ? 80 : 16 * BWV> {    // (4-bit value 
   }
 };
 
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void *src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() {
+  asm volatile("cp.async.commit_group;\n" ::: "memory");
+}
+template <int N> __device__ __forceinline__ void cp_async_wait() {
+  asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
+}
 // ---- asynchronous copies and their barriers -----------------------------------
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(bar), "r"(count) : "memory");
@@ -107,9 +136,161 @@ __device__ __forceinline__ void bulk_g2s(uint32_t dst, const void *src, uint32_t
       "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n"
       ::"r"(dst), "l"(src), "r"(bytes), "r"(bar) : "memory");
 }
+__device__ __forceinline__ void griddep_wait() {
+  asm volatile("griddepcontrol.wait;\n" ::: "memory");
+}
+__device__ __forceinline__ void griddep_launch() {
+  asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+}
+
 }  // namespace mma
 
 using namespace mma;
+
+// Value side of one tile: the lane holds coordinates 16g..16g+15 of tokens
+// 2t, 2t+1 (A, B) and 2t+8, 2t+9 (C, D); `at` = address of its 16 codes of
+// token 2t.  MMA j (0..7) takes coordinates 16g+2j (row g) and 16g+2j+1 (row
+// g+8) of the output tile.
+template <int BW, int VROW>
+__device__ __forceinline__ void value_mmas(uint32_t at, uint32_t sel, uint32_t pb0, uint32_t pb1,
+                                           float (&acc)[8][4]) {
+  constexpr int NB8 = 2 * BW;                       // bytes of 16 codes
+  if constexpr (BW == 4) {
+    const uint2 wa = lds64(at), wb = lds64(at + VROW);
+    const uint2 wc = lds64(at + 8 * VROW), wd = lds64(at + 9 * VROW);
+    // byte j of lo_* : low nibbles of tokens (A | B << 4) at coordinate 16g+2j
+    // byte j of hi_* : high nibbles, coordinate 16g+2j+1
+    auto up4 = [](uint32_t x) { return x << 4; };
+    auto down4 = [](uint32_t x) { return x >> 4; };
+    const uint32_t lo_ab[2] = {(wa.x & 0x0F0F0F0Fu) | (up4(wb.x) & 0xF0F0F0F0u),
+                               (wa.y & 0x0F0F0F0Fu) | (up4(wb.y) & 0xF0F0F0F0u)};
+    const uint32_t hi_ab[2] = {(down4(wa.x) & 0x0F0F0F0Fu) | (wb.x & 0xF0F0F0F0u),
+                               (down4(wa.y) & 0x0F0F0F0Fu) | (wb.y & 0xF0F0F0F0u)};
+    const uint32_t lo_cd[2] = {(wc.x & 0x0F0F0F0Fu) | (up4(wd.x) & 0xF0F0F0F0u),
+                               (wc.y & 0x0F0F0F0Fu) | (up4(wd.y) & 0xF0F0F0F0u)};
+    const uint32_t hi_cd[2] = {(down4(wc.x) & 0x0F0F0F0Fu) | (wd.x & 0xF0F0F0F0u),
+                               (down4(wc.y) & 0x0F0F0F0Fu) | (wd.y & 0xF0F0F0F0u)};
+    // The sixteen table addresses of a half are formed first, then the sixteen
+    // lookups are issued, then the four MMAs: a lookup never waits for the
+    // byte-permute that builds its own address.
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      uint32_t ad[4][4], f[4][4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const uint32_t src = q == 0 ? lo_ab[h] : q == 1 ? hi_ab[h] : q == 2 ? lo_cd[h] : hi_cd[h];
+        ad[0][q] = lut_addr<0>(src, sel); ad[1][q] = lut_addr<1>(src, sel);
+        ad[2][q] = lut_addr<2>(src, sel); ad[3][q] = lut_addr<3>(src, sel);
+      }
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+#pragma unroll
+        for (int q = 0; q < 4; ++q) f[j][q] = lds32(ad[j][q]);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) mma16816(acc[4 * h + j], f[j][0], f[j][1], f[j][2], f[j][3], pb0, pb1);
+    }
+  } else {
+    constexpr int NW = NB8 / 4;
+    uint32_t wa[NW], wb[NW], wc[NW], wd[NW];
+    load_words<NB8>(at, wa);
+    load_words<NB8>(at + VROW, wb);
+    load_words<NB8>(at + 8 * VROW, wc);
+    load_words<NB8>(at + 9 * VROW, wd);
+    auto one = [&](auto jc) {
+      constexpr int j = decltype(jc)::value;
+      mma16816(acc[j],
+               join(lut_code<BW, 2 * j>(wa, sel), lut_code<BW, 2 * j>(wb, sel)),
+               join(lut_code<BW, 2 * j + 1>(wa, sel), lut_code<BW, 2 * j + 1>(wb, sel)),
+               join(lut_code<BW, 2 * j>(wc, sel), lut_code<BW, 2 * j>(wd, sel)),
+               join(lut_code<BW, 2 * j + 1>(wc, sel), lut_code<BW, 2 * j + 1>(wd, sel)), pb0, pb1);
+    };
+    one(std::integral_constant<int, 0>{}); one(std::integral_constant<int, 1>{});
+    one(std::integral_constant<int, 2>{}); one(std::integral_constant<int, 3>{});
+    one(std::integral_constant<int, 4>{}); one(std::integral_constant<int, 5>{});
+    one(std::integral_constant<int, 6>{}); one(std::integral_constant<int, 7>{});
+  }
+}
+
+// Scores of one tile: S^T fragment (rows g, g+8; heads 2t, 2t+1), unscaled.
+// `at` = address of the lane's 32 codes of token row g.  Even and odd
+// contraction steps accumulate separately (two chains of four dependent MMAs
+// instead of one of eight).
+template <int BW>
+__device__ __forceinline__ void key_mmas(uint32_t at, uint32_t sel, const uint32_t (&qf)[8][2],
+                                         float (&c)[4]) {
+  constexpr int NB4 = 4 * BW;                       // bytes of 32 codes
+  constexpr int NW = NB4 / 4, NB = 16 * BW;
+  uint32_t w0[NW], w1[NW];
+  load_words<NB4>(at, w0);
+  load_words<NB4>(at + 8 * NB, w1);
+  constexpr int kChains = 2;
+  float cc[kChains][4];
+#pragma unroll
+  for (int i = 0; i < kChains; ++i) cc[i][0] = cc[i][1] = cc[i][2] = cc[i][3] = 0.f;
+  if constexpr (BW == 4) {
+    // per word of the two rows: eight addresses, eight lookups, two MMAs
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      uint32_t ad[8], f[8];
+      ad[0] = lut_addr<0>(w0[j], sel); ad[1] = lut_addr<0>(w1[j], sel);
+      ad[2] = lut_addr<1>(w0[j], sel); ad[3] = lut_addr<1>(w1[j], sel);
+      ad[4] = lut_addr<2>(w0[j], sel); ad[5] = lut_addr<2>(w1[j], sel);
+      ad[6] = lut_addr<3>(w0[j], sel); ad[7] = lut_addr<3>(w1[j], sel);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) f[i] = lds32(ad[i]);
+      mma16816(cc[0], f[0], f[1], f[2], f[3], qf[2 * j][0], qf[2 * j][1]);
+      mma16816(cc[1], f[4], f[5], f[6], f[7], qf[2 * j + 1][0], qf[2 * j + 1][1]);
+    }
+  } else {
+    auto one = [&](auto ksc) {
+      constexpr int ks = decltype(ksc)::value;
+      uint32_t a[4];
+      key_fragment<BW, ks>(w0, w1, sel, a);
+      mma16816(cc[ks % kChains], a[0], a[1], a[2], a[3], qf[ks][0], qf[ks][1]);
+    };
+    one(std::integral_constant<int, 0>{}); one(std::integral_constant<int, 1>{});
+    one(std::integral_constant<int, 2>{}); one(std::integral_constant<int, 3>{});
+    one(std::integral_constant<int, 4>{}); one(std::integral_constant<int, 5>{});
+    one(std::integral_constant<int, 6>{}); one(std::integral_constant<int, 7>{});
+  }
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    float v = cc[0][e];
+#pragma unroll
+    for (int i = 1; i < kChains; ++i) v += cc[i][e];
+    c[e] = v;
+  }
+}
+
+// fp32 scores of tile rows g and g+8 against two query rows (already rotated
+// and scaled, read through L1), times the key norms: {row g . qa, row g . qb,
+// row g+8 . qa, row g+8 . qb}.  Kept out of line: it runs only for windows
+// whose fp16 scores came out large, and must not cost the common path
+// registers.
+template <int BW>
+__device__ __noinline__ float4 precise_scores(uint32_t kbase, uint32_t nk_addr, int g,
+                                              const float *qa, const float *qb,
+                                              const float *centroids) {
+  constexpr int NB = 16 * BW;
+  float d0 = 0.f, d1 = 0.f, d2 = 0.f, d3 = 0.f;
+  const uint32_t r0 = kbase + g * NB, r1 = kbase + (g + 8) * NB;
+#pragma unroll 1
+  for (int d = 0; d < 128; ++d) {
+    const int bit = d * BW, b0 = bit >> 3, sh = bit & 7;
+    uint32_t x0 = lds_u8(r0 + b0), x1 = lds_u8(r1 + b0);
+    if (sh + BW > 8) {
+      x0 |= lds_u8(r0 + b0 + 1) << 8;
+      x1 |= lds_u8(r1 + b0 + 1) << 8;
+    }
+    const float c0 = __ldg(centroids + ((x0 >> sh) & ((1u << BW) - 1u)));
+    const float c1 = __ldg(centroids + ((x1 >> sh) & ((1u << BW) - 1u)));
+    const float fa = __ldg(qa + d), fb = __ldg(qb + d);
+    d0 = fmaf(fa, c0, d0); d1 = fmaf(fb, c0, d1);
+    d2 = fmaf(fa, c1, d2); d3 = fmaf(fb, c1, d3);
+  }
+  const float nk0 = lds_half(nk_addr + g * 2), nk1 = lds_half(nk_addr + (g + 8) * 2);
+  return make_float4(d0 * nk0, d1 * nk0, d2 * nk1, d3 * nk1);
+}
 
 template <int BWK, int BWV, bool S16>
 __global__ void __launch_bounds__(Cfg<BWK, BWV>::kThreads, 1)
@@ -350,33 +531,171 @@ decode_mma_kernel(DecodeParams p, int chunk_tokens) {
     ++fifo_r;
 
     // ---- query fragments: head g, coordinates 32t .. 32t+31 ----------------
-    ScanState<128> st;
-    const float *q0 = p.q_rot + ((int64_t)b * p.Hq + kvh * p.n_rep) * 128;
+    uint32_t qf[8][2];
     {
       const bool live = g < p.n_rep;
-      const float4 *src = reinterpret_cast<const float4 *>(q0 + (live ? g : 0) * 128 + 32 * t);
+      const float4 *src = reinterpret_cast<const float4 *>(
+          p.q_rot + ((int64_t)b * p.Hq + kvh * p.n_rep + (live ? g : 0)) * 128 + 32 * t);
 #pragma unroll
       for (int ks = 0; ks < 8; ++ks) {
         float4 v = live ? src[ks] : make_float4(0.f, 0.f, 0.f, 0.f);
-        st.qf[ks][0] = pack_half2(v.x, v.y);
-        st.qf[ks][1] = pack_half2(v.z, v.w);
+        qf[ks][0] = pack_half2(v.x, v.y);
+        qf[ks][1] = pack_half2(v.z, v.w);
       }
     }
-    st.clear();
+    float acc[8][4];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.f;
+    // Softmax state of heads 2t, 2t+1: reference M (the probabilities are
+    // 2^(s - M), M >= every score seen), -M with -inf replaced by 0, the bound
+    // a window's scores (relative to M) must stay under to take the short path,
+    // and the sum of the probabilities.
+    float M0 = -INFINITY, M1 = -INFINITY, neg0 = 0.f, neg1 = 0.f;
+    float hi0 = -INFINITY, hi1 = -INFINITY, l0 = 0.f, l1 = 0.f;
 
+    // A window whose 32 tokens all exist on pages that were found needs no
+    // masks; only the last window of a chunk (or a refused page id) takes the
+    // masked form of the same code.
     const int n_full = (tok1 - tok0) / kIterTokens;            // windows without a ragged end
     const int n_iter = (tok1 - tok0 + kIterTokens - 1) / kIterTokens;
     int wtok = tok0;                                           // first token of the window
+    uint32_t loaded = 3u;
+      auto window = [&](auto masked_c) {
+        constexpr bool MASKED = decltype(masked_c)::value;
+        const uint32_t slot0 = cbase;
+        // ---- scores of the tiles --------------------------------------------
+        float c[kTilesPerIter][4], a[kTilesPerIter][4], nk[kTilesPerIter][2];
+        bool ok[kTilesPerIter][2];
+#pragma unroll
+        for (int u = 0; u < kTilesPerIter; ++u) {
+          const uint32_t slot = slot0 + u * C::kSlot;
+          key_mmas<BWK>(slot + g * C::NBK + t * (4 * BWK), sel_k, qf, c[u]);
+          nk[u][0] = lds_half(slot + C::kOffNK + g * 2);
+          nk[u][1] = lds_half(slot + C::kOffNK + (g + 8) * 2);
+          ok[u][0] = ok[u][1] = true;
+        }
+        bool slow = true;
+        if constexpr (!MASKED) {
+          float top0 = -INFINITY, top1 = -INFINITY;
+#pragma unroll
+          for (int u = 0; u < kTilesPerIter; ++u) {
+            a[u][0] = fmaf(c[u][0], nk[u][0], neg0); a[u][1] = fmaf(c[u][1], nk[u][0], neg1);
+            a[u][2] = fmaf(c[u][2], nk[u][1], neg0); a[u][3] = fmaf(c[u][3], nk[u][1], neg1);
+            top0 = max3(top0, a[u][0], a[u][2]);
+            top1 = max3(top1, a[u][1], a[u][3]);
+          }
+          slow = __any_sync(kFull, top0 > hi0 || top1 > hi1);
+        }
+        if (slow) {
+          // A score above the reference (or the first window, a large score, a
+          // partly filled window): exact scores, fp32 rescoring when they are
+          // large, new reference, state rescaled.
+          float s[kTilesPerIter][4];
+          float big = 0.f;
+#pragma unroll
+          for (int u = 0; u < kTilesPerIter; ++u) {
+            s[u][0] = c[u][0] * nk[u][0]; s[u][1] = c[u][1] * nk[u][0];
+            s[u][2] = c[u][2] * nk[u][1]; s[u][3] = c[u][3] * nk[u][1];
+            if constexpr (MASKED) {
+              const int tok = wtok + u * kTileTokens;
+              const bool page_ok = (loaded >> u) & 1u;
+              ok[u][0] = page_ok && tok + g < tok1;
+              ok[u][1] = page_ok && tok + g + 8 < tok1;
+            }
+            if (ok[u][0]) big = fmaxf(big, fmaxf(fabsf(s[u][0]), fabsf(s[u][1])));
+            if (ok[u][1]) big = fmaxf(big, fmaxf(fabsf(s[u][2]), fabsf(s[u][3])));
+          }
+          // fp16 operands carry about 2^-11.5 of the score scale as error; when
+          // any score of this window is large (|s| > 8 in log2 units) its tiles
+          // are scored again in fp32 on the CUDA cores, so that large logits
+          // cost time, not accuracy.
+          if (__any_sync(kFull, big > kPreciseAbove)) {
+            const float *q0 = p.q_rot + ((int64_t)b * p.Hq + kvh * p.n_rep) * 128;
+            const bool h0 = 2 * t < p.n_rep, h1 = 2 * t + 1 < p.n_rep;
+            const float *qa = q0 + (h0 ? 2 * t : 0) * 128, *qb = q0 + (h1 ? 2 * t + 1 : 0) * 128;
+#pragma unroll
+            for (int u = 0; u < kTilesPerIter; ++u) {
+              const uint32_t slot = slot0 + u * C::kSlot;
+              const float4 d = precise_scores<BWK>(slot, slot + C::kOffNK, g, qa, qb, p.k.centroids);
+              s[u][0] = h0 ? d.x : 0.f; s[u][1] = h1 ? d.y : 0.f;
+              s[u][2] = h0 ? d.z : 0.f; s[u][3] = h1 ? d.w : 0.f;
+            }
+          }
+          float mx0 = -INFINITY, mx1 = -INFINITY;
+#pragma unroll
+          for (int u = 0; u < kTilesPerIter; ++u) {
+            if (!ok[u][0]) s[u][0] = s[u][1] = -INFINITY;
+            if (!ok[u][1]) s[u][2] = s[u][3] = -INFINITY;
+            mx0 = fmaxf(mx0, fmaxf(s[u][0], s[u][2]));
+            mx1 = fmaxf(mx1, fmaxf(s[u][1], s[u][3]));
+          }
+#pragma unroll
+          for (int o = 4; o < 32; o <<= 1) {
+            mx0 = fmaxf(mx0, __shfl_xor_sync(kFull, mx0, o));
+            mx1 = fmaxf(mx1, __shfl_xor_sync(kFull, mx1, o));
+          }
+          const float n0 = mx0 > M0 ? mx0 + kSlack : M0;
+          const float n1 = mx1 > M1 ? mx1 + kSlack : M1;
+          if (__any_sync(kFull, n0 != M0 || n1 != M1)) {
+            // 2^(-inf - x) = 0 for the first window; an unchanged reference keeps 1
+            const float alpha0 = n0 != M0 ? ex2(M0 - n0) : 1.f;
+            const float alpha1 = n1 != M1 ? ex2(M1 - n1) : 1.f;
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+              acc[j][0] *= alpha0; acc[j][1] *= alpha1; acc[j][2] *= alpha0; acc[j][3] *= alpha1;
+            }
+            l0 *= alpha0;
+            l1 *= alpha1;
+            M0 = n0;
+            M1 = n1;
+          }
+          // exp2(-inf - -inf) is defined as 0: with nothing seen the base is 0
+          neg0 = M0 == -INFINITY ? 0.f : -M0;
+          neg1 = M1 == -INFINITY ? 0.f : -M1;
+          // short path while every score stays under the reference and under the
+          // rescoring threshold; never when the running maximum is a large
+          // negative number (all scores are large then)
+          hi0 = (M0 == -INFINITY || M0 - kSlack < -kPreciseAbove) ? -INFINITY
+                                                                 : fminf(0.f, kPreciseAbove - M0);
+          hi1 = (M1 == -INFINITY || M1 - kSlack < -kPreciseAbove) ? -INFINITY
+                                                                 : fminf(0.f, kPreciseAbove - M1);
+#pragma unroll
+          for (int u = 0; u < kTilesPerIter; ++u) {
+            a[u][0] = s[u][0] + neg0; a[u][1] = s[u][1] + neg1;
+            a[u][2] = s[u][2] + neg0; a[u][3] = s[u][3] + neg1;
+          }
+        }
+
+        // ---- values of the tiles --------------------------------------------
+#pragma unroll
+        for (int u = 0; u < kTilesPerIter; ++u) {
+          const uint32_t slot = slot0 + u * C::kSlot;
+          const float nv0 = lds_half(slot + C::kOffNV + g * 2);
+          const float nv1 = lds_half(slot + C::kOffNV + (g + 8) * 2);
+          const float p0 = ex2(a[u][0]), p1 = ex2(a[u][1]);
+          const float p2 = ex2(a[u][2]), p3 = ex2(a[u][3]);
+          l0 += p0 + p2;
+          l1 += p1 + p3;
+          // rows g / g+8 of P' (token x head) -> B fragment (token pairs of head g)
+          uint32_t r0 = pack_half2(p0 * nv0, p1 * nv0), r1 = pack_half2(p2 * nv1, p3 * nv1);
+          if constexpr (MASKED) {
+            r0 = ok[u][0] ? r0 : 0u;
+            r1 = ok[u][1] ? r1 : 0u;
+          }
+          const uint32_t pb0 = movmatrix_trans(r0), pb1 = movmatrix_trans(r1);
+          value_mmas<BWV, C::kVRow>(slot + C::kOffV + g * (2 * BWV) + (2 * t) * C::kVRow, sel_v, pb0,
+                                    pb1, acc);
+        }
+      };
     for (int it = 0; it < n_iter; ++it) {
       issue_one();
       cp_async_wait<1>();
       __syncwarp();
       if (it < n_full && bad == 0u) {
-        scan_window<typename C::Base, false>(st, cbase, wtok, tok1, 3u, g, t, sel_k, sel_v, q0, p.n_rep,
-                                             p.k.centroids);
+        window(std::false_type{});
       } else {
-        scan_window<typename C::Base, true>(st, cbase, wtok, tok1, ~(bad >> (2 * chalf)) & 3u, g, t, sel_k,
-                                            sel_v, q0, p.n_rep, p.k.centroids);
+        loaded = ~(bad >> (2 * chalf)) & 3u;
+        window(std::true_type{});
       }
       __syncwarp();       // every lane is done with this half of the ring before it is refilled
       cbase = 2 * ring + kTilesPerIter * C::kSlot - cbase;
@@ -387,8 +706,8 @@ decode_mma_kernel(DecodeParams p, int chunk_tokens) {
     // ---- partial state of this chunk ---------------------------------------
 #pragma unroll
     for (int o = 4; o < 32; o <<= 1) {
-      st.l0 += __shfl_xor_sync(kFull, st.l0, o);
-      st.l1 += __shfl_xor_sync(kFull, st.l1, o);
+      l0 += __shfl_xor_sync(kFull, l0, o);
+      l1 += __shfl_xor_sync(kFull, l1, o);
     }
 #pragma unroll
     for (int e = 0; e < 2; ++e) {
@@ -397,10 +716,10 @@ decode_mma_kernel(DecodeParams p, int chunk_tokens) {
         const int64_t row = ((int64_t)b * p.Hq + kvh * p.n_rep + h) * chunks + chunk;
         float2 *dst = reinterpret_cast<float2 *>(p.part_acc + row * 128 + 16 * g);
 #pragma unroll
-        for (int j = 0; j < 8; ++j) dst[j] = make_float2(st.acc[j][e], st.acc[j][2 + e]);
+        for (int j = 0; j < 8; ++j) dst[j] = make_float2(acc[j][e], acc[j][2 + e]);
         if (g == 0) {
-          p.part_m[row] = e ? st.M1 : st.M0;
-          p.part_l[row] = e ? st.l1 : st.l0;
+          p.part_m[row] = e ? M1 : M0;
+          p.part_l[row] = e ? l1 : l0;
         }
       }
     }

@@ -1,8 +1,7 @@
-// The page scan of the tensor-core decode kernels at head_dim 128, in the parts
-// their two schedules share: how a 16-token tile lies in shared memory, the
-// fragments of the score and value MMAs built from packed codes, and one 32-token
-// window of the online softmax.  Used by wtq_decode_mma.cu (split-K over all
-// multiprocessors) and wtq_decode_fused.cu (one launch per call).
+// The page scan of the one-launch decode kernel (wtq_decode_fused.cu): how a 16-token
+// tile lies in shared memory, and at head_dim 128 the fragments of the score and value
+// MMAs built from packed codes and one 32-token window of the online softmax, by the
+// steps of the split-K scan (wtq_decode_mma.cu, which keeps its own: see there).
 #pragma once
 
 #include <type_traits>
