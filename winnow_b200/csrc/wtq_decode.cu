@@ -20,8 +20,8 @@
 
 namespace wtq {
 
-// The rotation may be scheduled while the kernel ahead of it drains (an append, the
-// merge of the previous call).  Until the wait it reads nothing but Pi; after it,
+// A small rotation may be scheduled while the kernel ahead of it drains (an append, the
+// merge of the previous call; see launch_rotate_q).  Until the wait it reads nothing but Pi; after it,
 // every kernel ahead has completed, and only then are the scan's blocks let in, so
 // that the scan too may read pages, table and lengths before its own wait.
 __device__ __forceinline__ void begin_rotation() {
@@ -546,7 +546,12 @@ int launch_rotate_q(const void *q, int dtype, const int64_t *qs, const float *Pi
   cfg.blockDim = dim3(kRotThreads);
   cfg.stream = stream;
   cfg.attrs = &pdl;
-  cfg.numAttrs = 1;
+  // Under the tail of the kernel ahead only where the rotation is small: its blocks' reads of
+  // Pi compete with that kernel for L2, which behind a merge costs more than the head start
+  // gives (plain / overlapped, us a call among others: 64 rows 59.4 / 58.0, 96 rows 23.3 / 22.3,
+  // 192 rows 21.8 / 21.1; 512 rows 54.9 / 56.3, 1024 rows behind an append 260.0 / 262.3,
+  // 2048 rows 60.6 / 62.8).
+  cfg.numAttrs = rows <= 256 ? 1 : 0;
   cudaError_t e;
   auto fixed = [&](auto kernel, int nr, int most) {            // head_dim 128
     cfg.gridDim = dim3((unsigned)std::min((rows + nr - 1) / nr, most));
